@@ -922,7 +922,7 @@ def main():
     achieved = (total_bytes + state_bytes) / (ms * 1e-3) / 1e9
     chosen = [l for l in tune_report.splitlines() if l.startswith("chosen:")]
     kernel = (chosen[0][len("chosen:"):].split(", chunk=")[0].strip() if chosen else
-              "k_batch32xk<%d>%s" % (plan_cfg["core"], " after k_jump_part5 (%d windows jumped "
+              "k_batch32xk<%d>%s" % (plan_cfg["core"], " after k_jump_part (%d windows jumped "
                                      "ahead)" % plan_cfg["prejumps"] if plan_cfg["prejumps"] else ""))
     # DRAM bytes (read + write) per step of the plan's kernels, from an ncu
     # capture of the same plan on the same workload (profiles/); reported

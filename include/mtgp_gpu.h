@@ -435,10 +435,10 @@ int mtgp_gpu_plan_describe(const mtgp_gpu_plan_t *plan, int64_t *values,
  *   "single_chunk" chunk length of a split single-generator fill (fills of
  *                  at least 2^20 values): 0 = automatic, > 0 = that length
  *   "jump_parts"   jumps made ahead of a batched launch (the chunk starts of
- *                  such a fill, and batched tasks that start with one jump):
- *                  CTAs per jump, 0 = automatic (4), > 0 = that many (at
- *                  most one per tap chunk of the jump kernel); -1 = such
- *                  jumps run inside the batched kernel instead
+ *                  such a fill, and batched tasks that start with a jump):
+ *                  CTAs per jump, 0 = automatic (1 to 8, by the number of
+ *                  jumps), > 0 = that many (at most 32); -1 = such jumps run
+ *                  inside the batched kernel instead
  *   "jump_overlap" 0 = the jump parts run before the persistent launch;
  *                  1 = they run on a side stream of the plan, followed there
  *                  by a second persistent launch of the tasks that start

@@ -58,9 +58,9 @@ constexpr uint64_t kMaxGenSkip = uint64_t(1) << 34;
 
 // single_chunk: chunk length of split single-generator fills (0 =
 // automatic).  jump_parts: CTAs per jump made ahead of a batched launch
-// (split single fills, and batched tasks that start with one jump): 0 =
-// four, at most one per tap chunk of the jump kernel; -1 = such jumps run
-// inside the batched kernel instead.
+// (split single fills, and batched tasks that start with a jump): 0 =
+// automatic, at most kJumpUnits; -1 = such jumps run inside the batched
+// kernel instead.
 // core: the 32-bit generation core (2 = two words per thread, 4 = four, 1
 // = one); poly_window: bits per comb window of the GPU's polynomial
 // products (0 = automatic, 2, 4).  Every pool and single generator carries
@@ -119,16 +119,16 @@ inline int applyTuning(Tuning &t, const char *key, int64_t value) {
     return MTGP_OK;
 }
 
-// Jumps made ahead of a batched launch run as four CTAs each: every part
-// regenerates the sequence up to its taps, so one CTA per tap chunk (11 for
-// MEXP 11213) costs more than it saves (measured on split single fills).
-constexpr int kJumpParts = 4;
-
-// CTAs per jump made ahead of a batched launch, for a jump of tchunks tap
-// chunks (tuning knob jump_parts).
-inline int jumpParts(const Tuning &t, int tchunks) {
-    const int64_t p = t.jump_parts > 0 ? t.jump_parts : kJumpParts;
-    return (int)std::min<int64_t>(p, tchunks);
+// CTAs per jump, for njumps jumps made together ahead of a batched launch
+// (tuning knob jump_parts; automatic: as many as keep all the jumps' CTAs
+// resident at once, two per SM, and at most eight).  Every part makes the
+// sequence anew, so more parts than that only add work: one generator's fill
+// of 2^20 values (31 jumps) takes 36 us with 4 to 8 parts, 42 with 16; 255
+// jumps at MEXP 11213/64 take 32 us with one part, 49 with three.
+constexpr int kMaxJumpParts = 8;
+inline int jumpParts(const Tuning &t, int njumps, int sms) {
+    if (t.jump_parts > 0) return (int)std::min<int64_t>(t.jump_parts, kJumpUnits);
+    return std::max(1, std::min(kMaxJumpParts, 2 * sms / std::max(1, njumps)));
 }
 
 // ------------------------------------------------------------------------
@@ -160,7 +160,6 @@ struct T32 {
                              W *dst, int stride, const JumpPart *d, int nd, cudaStream_t s) {
         return launchJumpParts32(mexp, p, st, polys, nw, dst, stride, d, nd, s);
     }
-    static int jumpChunks(int mexp, int nw) { return jumpChunks32(mexp, nw); }
     static cudaError_t windows(const W *gen, W *win, int n, int stride, int nwin, cudaStream_t s) {
         return launchChunkWindows32(gen, win, n, stride, nwin, s);
     }
@@ -210,7 +209,6 @@ struct T64 {
                              W *dst, int stride, const JumpPart *d, int nd, cudaStream_t s) {
         return launchJumpParts64(mexp, p, st, polys, nw, dst, stride, d, nd, s);
     }
-    static int jumpChunks(int mexp, int nw) { return jumpChunks64(mexp, nw); }
     static cudaError_t windows(const W *gen, W *win, int n, int stride, int nwin, cudaStream_t s) {
         return launchChunkWindows64(gen, win, n, stride, nwin, s);
     }

@@ -193,17 +193,18 @@ struct JumpDesc {
     uint64_t src;      // element offset of the source window
     uint64_t dst;      // element offset of the destination window
 };
-// Partial jumps: CTA b correlates the tap chunks [ch0, ch1) of one jump and
-// XORs the result into its destination window (zero on entry); the parts of
-// a jump together give the full jump.  jumpChunks*() = tap chunks of one
-// jump.  Source windows are in `states`, polynomials in `polys` (nwords
-// words each), destination windows `stride` words apart from `dst`.
+// Partial jumps: CTA b correlates the share [u0, u1) of kJumpUnits of one
+// jump's taps and XORs the result into its destination window (zero on
+// entry); the parts of a jump together give the full jump.  Source windows
+// are in `states`, polynomials in `polys` (nwords words each), destination
+// windows `stride` words apart from `dst`.
+constexpr int kJumpUnits = 32;
 struct JumpPart {
     uint64_t src;      // element offset of the source window in states
     int32_t poly;      // polynomial index
     int32_t dst;       // destination window index
     int32_t pidx;      // parameter-set index
-    int16_t ch0, ch1;
+    int16_t u0, u1;
 };
 static_assert(sizeof(JumpPart) == 24, "JumpPart is 24 bytes");
 cudaError_t launchJumpParts32(int mexp, const DevParams32 *params, const uint32_t *states,
@@ -212,8 +213,6 @@ cudaError_t launchJumpParts32(int mexp, const DevParams32 *params, const uint32_
 cudaError_t launchJumpParts64(int mexp, const DevParams64 *params, const uint64_t *states,
                               const uint32_t *polys, int nwords, uint64_t *dst, int stride,
                               const JumpPart *parts, int nparts, cudaStream_t s);
-int jumpChunks32(int mexp, int nwords);
-int jumpChunks64(int mexp, int nwords);
 // nwin windows of `stride` words at win: window 0 = gen[0..n), the others
 // zero (the destinations of jump parts).
 cudaError_t launchChunkWindows32(const uint32_t *gen, uint32_t *win, int n, int stride, int nwin,

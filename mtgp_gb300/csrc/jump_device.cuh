@@ -84,88 +84,17 @@ __device__ __forceinline__ void ringPut(W *ring, uint32_t k, W v) {
     if (k < (uint32_t)Geo::MIR) ring[Geo::RING + k] = v;
 }
 
-// The taps of one group, J .. J+3, against the lane's R outputs: bit t of
-// D says whether tap J + t is set.  Tap J + t reads seq[base + J + t + r]
-// for output r: win[(J + t + r) % R] while t + r < R (the register window,
-// rotated), else nx[t + r - R], the words just past the window.  The terms
-// are XOR-ed in a chain that the compiler fuses into three-input XORs (two
-// terms per instruction).
-template <class Tr, int R, int J, int D>
-__device__ __forceinline__ void tapGroup(typename Tr::W (&acc)[R], const typename Tr::W (&win)[R],
-                                         const typename Tr::W (&nx)[4]) {
-    using W = typename Tr::W;
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-        W v = acc[r];
-#pragma unroll
-        for (int t = 0; t < 4; t++)
-            if ((D >> t) & 1) v ^= (t + r < R) ? win[(J + t + r) % R] : nx[t + r - R];
-        acc[r] = v;
-    }
-}
-
-// One uniform branch per group of NT4 <= 4 taps: the group's coefficient
-// bits are the same for the whole warp.
-template <class Tr, int R, int J, int NT4>
-__device__ __forceinline__ void tapSwitch(typename Tr::W (&acc)[R], const typename Tr::W (&win)[R],
-                                          const typename Tr::W (&nx)[4], uint32_t d) {
-#define MTGP_TAP_CASE(D) \
-    case D:              \
-        if constexpr ((D >> NT4) == 0) tapGroup<Tr, R, J, D>(acc, win, nx); \
-        break;
-    switch (d) {
-        MTGP_TAP_CASE(1) MTGP_TAP_CASE(2) MTGP_TAP_CASE(3) MTGP_TAP_CASE(4)
-        MTGP_TAP_CASE(5) MTGP_TAP_CASE(6) MTGP_TAP_CASE(7) MTGP_TAP_CASE(8)
-        MTGP_TAP_CASE(9) MTGP_TAP_CASE(10) MTGP_TAP_CASE(11) MTGP_TAP_CASE(12)
-        MTGP_TAP_CASE(13) MTGP_TAP_CASE(14) MTGP_TAP_CASE(15)
-    default: break;
-    }
-#undef MTGP_TAP_CASE
-}
-
-// Groups J, J + 4, ... of the R taps of one tapsR call; each group's words
-// replace the window words its taps no longer need.
-template <class Tr, int R, int J>
-__device__ __forceinline__ void tapGroups(typename Tr::W (&acc)[R], typename Tr::W (&win)[R],
-                                          const typename Tr::W *rp, uint32_t bits_lo,
-                                          uint32_t bits_hi) {
-    if constexpr (J < R) {
-        using W = typename Tr::W;
-        constexpr int NT4 = R - J < 4 ? R - J : 4;
-        const uint32_t bj = J < 32 ? bits_lo : bits_hi;  // J % 4 == 0: never straddles bit 31
-        const uint32_t d = (bj >> (J & 31)) & ((1u << NT4) - 1u);
-        W nx[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) nx[u] = u < NT4 ? rp[R + J + u] : W(0);
-        tapSwitch<Tr, R, J, NT4>(acc, win, nx, d);
-#pragma unroll
-        for (int u = 0; u < NT4; u++) win[J + u] = nx[u];
-        tapGroups<Tr, R, J + 4>(acc, win, rp, bits_lo, bits_hi);
-    }
-}
-
-// Largest R for which taps go in groups of four (a 16-way branch per group,
-// whose code grows with R); larger R take them in pairs.  Groups of four
-// hold a few more registers live, so the jumps inside the batched kernels
-// (whose generation core caps the registers) keep pairs.
-constexpr int kQuadTapsMaxR = 13;
-
 // R taps p .. p+R-1 against the lane's R outputs: win holds seq[p + l0 ..
 // + R) on entry (l0 folded into base = p + l0) and the next R words on exit.
 // rp = ring + (base & (RING - 1)): the next R words are rp[R .. 2R), which
 // the mirror keeps contiguous, so every load is one base plus a constant.
-// The coefficients of a group of taps are the same for the whole warp, so
-// each group takes one uniform branch.  In groups of four, a set of m taps
-// costs ceil(m / 2) three-input XORs per output (1.25 per group on random
-// polynomials, 0.31 per tap); in pairs (larger R) 0.375 per tap.
-template <class Tr, class Geo, bool GROUPS4>
+// The coefficients of a pair of taps are the same for the whole warp, so each
+// pair takes one uniform branch.
+template <class Tr, class Geo>
 __device__ __forceinline__ void tapsR(typename Tr::W (&acc)[Geo::R], typename Tr::W (&win)[Geo::R],
                                       const typename Tr::W *rp, uint32_t bits_lo,
                                       uint32_t bits_hi) {
     constexpr int R = Geo::R;
-    if constexpr (GROUPS4 && R <= kQuadTapsMaxR) {
-        tapGroups<Tr, R, 0>(acc, win, rp, bits_lo, bits_hi);
-    } else {
 #pragma unroll
     for (int j = 0; j < R; j += 2) {  // j even: a pair never straddles bit 31
         const uint32_t bj = j < 32 ? bits_lo : bits_hi;
@@ -196,14 +125,13 @@ __device__ __forceinline__ void tapsR(typename Tr::W (&acc)[Geo::R], typename Tr
             win[j] = rp[R + j];
         }
     }
-    }
 }
 
 // Jump the window jin[0..N) in place by chain[0], chain[1], ... (uint32-array
 // polynomials of nwords words).  smem must hold Geo::bytes<W>(nwords) bytes
 // laid out as described above (jin first).  All NT threads must call it; it
-// begins and ends with a barrier.  GROUPS4: taps in groups of four (tapsR).
-template <class Tr, class Geo, bool GROUPS4, class ChainAt>
+// begins and ends with a barrier.
+template <class Tr, class Geo, class ChainAt>
 __device__ __forceinline__ void jump_chain_impl(typename Tr::W *smem, const typename Tr::Lane &L,
                                                 ChainAt chain, int nchain, int nwords) {
     using W = typename Tr::W;
@@ -256,7 +184,7 @@ __device__ __forceinline__ void jump_chain_impl(typename Tr::W *smem, const type
                     const uint32_t bits_hi =
                         R > 32 ? __funnelshift_r(poly[(p >> 5) + 1], poly[(p >> 5) + 2], p & 31)
                                : 0u;
-                    tapsR<Tr, Geo, GROUPS4>(acc, win, ring + ((uint32_t)(p + l0) & M), bits_lo, bits_hi);
+                    tapsR<Tr, Geo>(acc, win, ring + ((uint32_t)(p + l0) & M), bits_lo, bits_hi);
                 }
                 __syncthreads();
             }
@@ -273,14 +201,7 @@ __device__ __forceinline__ void jump_chain_impl(typename Tr::W *smem, const type
 template <class Tr, class Geo>
 __device__ void jump_chain(typename Tr::W *smem, const typename Tr::Lane &L,
                            const uint32_t *const *chain, int nchain, int nwords) {
-    jump_chain_impl<Tr, Geo, true>(smem, L, [chain](int c) { return chain[c]; }, nchain, nwords);
-}
-
-// One polynomial.
-template <class Tr, class Geo>
-__device__ void jump_one(typename Tr::W *smem, const typename Tr::Lane &L, const uint32_t *poly,
-                         int nwords) {
-    jump_chain_impl<Tr, Geo, true>(smem, L, [poly](int) { return poly; }, 1, nwords);
+    jump_chain_impl<Tr, Geo>(smem, L, [chain](int c) { return chain[c]; }, nchain, nwords);
 }
 
 // Part of one jump: the correlation over the tap chunks [ch0, ch1) only
@@ -333,7 +254,7 @@ __device__ void jump_part(typename Tr::W *smem, const typename Tr::Lane &L, cons
                     const uint32_t bits_hi =
                         R > 32 ? __funnelshift_r(poly[(p >> 5) + 1], poly[(p >> 5) + 2], p & 31)
                                : 0u;
-                    tapsR<Tr, Geo, true>(acc, win, ring + ((uint32_t)(p + l0) & M), bits_lo, bits_hi);
+                    tapsR<Tr, Geo>(acc, win, ring + ((uint32_t)(p + l0) & M), bits_lo, bits_hi);
                 }
             }
             __syncthreads();

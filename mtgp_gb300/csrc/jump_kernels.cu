@@ -1,22 +1,63 @@
 // jump_kernels.cu -- jump-ahead of many windows, one CTA per descriptor.
 //
 // Each descriptor names a source window, a destination window and a chain
-// of polynomials (jump_device.cuh).  Substream j of the reference's CUDA
+// of polynomials (jump_sorted.cuh).  Substream j of the reference's CUDA
 // sample is reached the same way, from the table of X^(4^k * 3^162) mod chi
 // (cuda-sample/mtgp32-jump-kernel.cuh:383-401), but there one thread steps
 // the recursion for every coefficient; here the whole CTA does.
-#include "jump_device.cuh"
+#include "jump_sorted.cuh"
 
 namespace mtgp {
 
 namespace {
 
-constexpr int kJumpThreads = 256;
+template <class G>
+__global__ void __launch_bounds__(G::NT, G::MINB)
+k_jump(const typename G::Tr::P *__restrict__ params, typename G::W *__restrict__ states,
+       const JumpDesc *__restrict__ descs, int nwords) {
+    using W = typename G::W;
+    extern __shared__ __align__(16) unsigned char smem[];
+    W *seq = reinterpret_cast<W *>(smem);
+    const W *jout = reinterpret_cast<const W *>(smem + G::off_jout);
+    const JumpDesc &D = descs[blockIdx.x];
+    typename G::Tr::Lane L;
+    L.load(params[D.pidx], threadIdx.x & 31);
+    for (int k = threadIdx.x; k < G::N; k += G::NT) seq[k] = states[D.src + k];
+    for (int c = 0; c < D.nchain; c++) {
+        jumpSorted<G>(smem, L, D.poly[c], nwords, 0, kJumpUnits);
+        for (int k = threadIdx.x; k < G::N; k += G::NT) seq[k] = jout[k];
+    }
+    for (int k = threadIdx.x; k < G::N; k += G::NT) states[D.dst + k] = seq[k];
+}
 
+// One CTA per (jump, share of its rows): XOR-ed into the zeroed destination
+// window.
+template <class G>
+__global__ void __launch_bounds__(G::NT, G::MINB)
+k_jump_part(const typename G::Tr::P *__restrict__ params, const typename G::W *__restrict__ states,
+            const uint32_t *__restrict__ polys, int nwords, typename G::W *__restrict__ dst,
+            int stride, const JumpPart *__restrict__ parts) {
+    using W = typename G::W;
+    extern __shared__ __align__(16) unsigned char smem[];
+    W *seq = reinterpret_cast<W *>(smem);
+    const W *jout = reinterpret_cast<const W *>(smem + G::off_jout);
+    const JumpPart &D = parts[blockIdx.x];
+    typename G::Tr::Lane L;
+    L.load(params[D.pidx], threadIdx.x & 31);
+    for (int k = threadIdx.x; k < G::N; k += G::NT) seq[k] = states[D.src + k];
+    jumpSorted<G>(smem, L, polys + (size_t)D.poly * nwords, nwords, D.u0, D.u1);
+    W *to = dst + (size_t)D.dst * stride;
+    for (int k = threadIdx.x; k < G::N; k += G::NT) G::Tr::axor(&to[k], jout[k]);
+}
+
+// The longer exponents: the taps unsorted, against a ring that holds part of
+// the sequence (jump_device.cuh).  An early form of the sorted kernel did not
+// end at MEXP 44497, although the same code does when its threads are run on
+// the CPU; the cause is not known, so it stays off there.
 template <class Tr, class Geo>
 __global__ void __launch_bounds__(Geo::NT)
-k_jump(const typename Tr::P *__restrict__ params, typename Tr::W *__restrict__ states,
-       const JumpDesc *__restrict__ descs, int nwords) {
+k_jump_ring(const typename Tr::P *__restrict__ params, typename Tr::W *__restrict__ states,
+            const JumpDesc *__restrict__ descs, int nwords) {
     using W = typename Tr::W;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     W *smem = reinterpret_cast<W *>(smem_raw);
@@ -28,14 +69,13 @@ k_jump(const typename Tr::P *__restrict__ params, typename Tr::W *__restrict__ s
     for (int k = threadIdx.x; k < Geo::N; k += Geo::NT) states[D.dst + k] = smem[k];
 }
 
-// One CTA per (jump, range of tap chunks): partial correlation XOR-ed into
-// the zeroed destination window (jump_device.cuh: jump_part).
+// A share [u0, u1) of kJumpUnits here is a range of whole chunks of taps.
 template <class Tr, class Geo>
-__device__ __forceinline__ void jumpPart(const typename Tr::P *__restrict__ params,
-                                         const typename Tr::W *__restrict__ states,
-                                         const uint32_t *__restrict__ polys, int nwords,
-                                         typename Tr::W *__restrict__ dst, int stride,
-                                         const JumpPart *__restrict__ parts) {
+__global__ void __launch_bounds__(Geo::NT)
+k_jump_part_ring(const typename Tr::P *__restrict__ params,
+                 const typename Tr::W *__restrict__ states, const uint32_t *__restrict__ polys,
+                 int nwords, typename Tr::W *__restrict__ dst, int stride,
+                 const JumpPart *__restrict__ parts) {
     using W = typename Tr::W;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     W *smem = reinterpret_cast<W *>(smem_raw);
@@ -44,84 +84,81 @@ __device__ __forceinline__ void jumpPart(const typename Tr::P *__restrict__ para
     L.load(params[D.pidx], threadIdx.x & 31);
     for (int k = threadIdx.x; k < Geo::N; k += Geo::NT) smem[k] = states[D.src + k];
     __syncthreads();
-    jump_part<Tr, Geo>(smem, L, polys + (size_t)D.poly * nwords, nwords, D.ch0, D.ch1,
+    const int chunks = (nwords * 32 + Geo::C - 1) / Geo::C;
+    jump_part<Tr, Geo>(smem, L, polys + (size_t)D.poly * nwords, nwords,
+                       chunks * D.u0 / kJumpUnits, chunks * D.u1 / kJumpUnits,
                        dst + (size_t)D.dst * stride);
 }
 
 template <class Tr, class Geo>
-__global__ void __launch_bounds__(Geo::NT)
-k_jump_part(const typename Tr::P *__restrict__ params, const typename Tr::W *__restrict__ states,
-            const uint32_t *__restrict__ polys, int nwords, typename Tr::W *__restrict__ dst,
-            int stride, const JumpPart *__restrict__ parts) {
-    jumpPart<Tr, Geo>(params, states, polys, nwords, dst, stride, parts);
-}
+struct Ring {};  // selects the unsorted kernels
 
-// The same with at most 48 registers, five CTAs per SM, for the 32-bit
-// geometries with groups of four taps: a bench step's 184 jumps × 4 parts
-// then run in one wave on 152 SMs (49 registers allowed four CTAs per SM,
-// 1.2 waves).
 template <class Tr, class Geo>
-__global__ void __launch_bounds__(Geo::NT, 5)
-k_jump_part5(const typename Tr::P *__restrict__ params, const typename Tr::W *__restrict__ states,
-             const uint32_t *__restrict__ polys, int nwords, typename Tr::W *__restrict__ dst,
-             int stride, const JumpPart *__restrict__ parts) {
-    jumpPart<Tr, Geo>(params, states, polys, nwords, dst, stride, parts);
-}
-
-template <class Tr, class Geo, class K>
-cudaError_t launchPartsWith(K kern, const typename Tr::P *params, const typename Tr::W *states,
-                            const uint32_t *polys, int nwords, typename Tr::W *dst, int stride,
-                            const JumpPart *parts, int nparts, cudaStream_t s) {
-    using W = typename Tr::W;
-    const size_t smem = Geo::template bytes<W>(nwords);
+cudaError_t launchParts(Ring<Tr, Geo>, const typename Tr::P *params, const typename Tr::W *states,
+                        const uint32_t *polys, int nwords, typename Tr::W *dst, int stride,
+                        const JumpPart *parts, int nparts, cudaStream_t s) {
+    const size_t smem = Geo::template bytes<typename Tr::W>(nwords);
     static std::atomic<size_t> seen[16];
-    cudaError_t e = allowSmem(kern, smem, seen);
+    cudaError_t e = allowSmem(k_jump_part_ring<Tr, Geo>, smem, seen);
     if (e != cudaSuccess) return e;
     if (nparts <= 0) return cudaSuccess;
-    kern<<<nparts, Geo::NT, smem, s>>>(params, states, polys, nwords, dst, stride, parts);
+    k_jump_part_ring<Tr, Geo><<<nparts, Geo::NT, smem, s>>>(params, states, polys, nwords, dst,
+                                                            stride, parts);
     return cudaGetLastError();
 }
 
 template <class Tr, class Geo>
-cudaError_t launchParts(const typename Tr::P *params, const typename Tr::W *states,
-                        const uint32_t *polys, int nwords, typename Tr::W *dst, int stride,
-                        const JumpPart *parts, int nparts, cudaStream_t s) {
-    if constexpr (sizeof(typename Tr::W) == 4 && Geo::R <= kQuadTapsMaxR)
-        return launchPartsWith<Tr, Geo>(k_jump_part5<Tr, Geo>, params, states, polys, nwords, dst,
-                                        stride, parts, nparts, s);
-    else
-        return launchPartsWith<Tr, Geo>(k_jump_part<Tr, Geo>, params, states, polys, nwords, dst,
-                                        stride, parts, nparts, s);
-}
-
-template <class Geo>
-int chunksOf(int nwords) { return (nwords * 32 + Geo::C - 1) / Geo::C; }
-
-template <class Tr, class Geo>
-cudaError_t launch(const typename Tr::P *params, typename Tr::W *states,
+cudaError_t launch(Ring<Tr, Geo>, const typename Tr::P *params, typename Tr::W *states,
                    const JumpDesc *descs, int ndesc, int nwords, cudaStream_t s) {
-    using W = typename Tr::W;
-    const size_t smem = Geo::template bytes<W>(nwords);
-    auto kern = k_jump<Tr, Geo>;
+    const size_t smem = Geo::template bytes<typename Tr::W>(nwords);
     static std::atomic<size_t> seen[16];
-    cudaError_t e = allowSmem(kern, smem, seen);
+    cudaError_t e = allowSmem(k_jump_ring<Tr, Geo>, smem, seen);
     if (e != cudaSuccess) return e;
     if (ndesc <= 0) return cudaSuccess;
-    kern<<<ndesc, Geo::NT, smem, s>>>(params, states, descs, nwords);
+    k_jump_ring<Tr, Geo><<<ndesc, Geo::NT, smem, s>>>(params, states, descs, nwords);
+    return cudaGetLastError();
+}
+
+template <class G>
+cudaError_t launchParts(G, const typename G::Tr::P *params, const typename G::W *states,
+                        const uint32_t *polys, int nwords, typename G::W *dst, int stride,
+                        const JumpPart *parts, int nparts, cudaStream_t s) {
+    static std::atomic<size_t> seen[16];
+    cudaError_t e = allowSmem(k_jump_part<G>, G::kBytes, seen);
+    if (e != cudaSuccess) return e;
+    if (nparts <= 0) return cudaSuccess;
+    k_jump_part<G><<<nparts, G::NT, G::kBytes, s>>>(params, states, polys, nwords, dst, stride,
+                                                    parts);
+    return cudaGetLastError();
+}
+
+template <class G>
+cudaError_t launch(G, const typename G::Tr::P *params, typename G::W *states, const JumpDesc *descs,
+                   int ndesc, int nwords, cudaStream_t s) {
+    static std::atomic<size_t> seen[16];
+    cudaError_t e = allowSmem(k_jump<G>, G::kBytes, seen);
+    if (e != cudaSuccess) return e;
+    if (ndesc <= 0) return cudaSuccess;
+    k_jump<G><<<ndesc, G::NT, G::kBytes, s>>>(params, states, descs, nwords);
     return cudaGetLastError();
 }
 
 }  // namespace
 
-#define MTGP_JGEO32(X)                                     \
-    X(11213, (JGeo<351, 11, kJumpThreads, 256, 2048>))     \
-    X(23209, (JGeo<726, 23, kJumpThreads, 256, 4096>))     \
-    X(44497, (JGeo<1391, 45, kJumpThreads, 256, 4096>))
-#define MTGP_JGEO64(X)                                     \
-    X(11213, (JGeo<176, 7, kJumpThreads, 128, 2048>))      \
-    X(23209, (JGeo<363, 13, kJumpThreads, 256, 2048>))     \
-    X(44497, (JGeo<696, 23, kJumpThreads, 256, 4096>))     \
-    X(110503, (JGeo<1727, 27, kJumpThreads, 256, 4096>))
+// Per exponent: live words, row ranges per CTA, words per recursion step,
+// taps per chunk, CTAs per SM.  The chunk is the whole polynomial where the
+// sequence then leaves room for two or three CTAs per SM, half of it at
+// MEXP 23209.
+constexpr int kRingThreads = 256;
+#define MTGP_JGEO32(X)                                              \
+    X(11213, (SJump<Tr32, 351, 4, 256, 11264, 2>))                  \
+    X(23209, (SJump<Tr32, 726, 2, 256, 11648, 2>))                  \
+    X(44497, (Ring<Tr32, JGeo<1391, 45, kRingThreads, 256, 4096>>))
+#define MTGP_JGEO64(X)                                              \
+    X(11213, (SJump<Tr64, 176, 4, 128, 11264, 2>))                  \
+    X(23209, (SJump<Tr64, 363, 2, 256, 11648, 2>))                  \
+    X(44497, (Ring<Tr64, JGeo<696, 23, kRingThreads, 256, 4096>>))  \
+    X(110503, (Ring<Tr64, JGeo<1727, 27, kRingThreads, 256, 4096>>))
 
 template <class G> struct Unwrap;
 template <class G> struct Unwrap<void(G)> { using T = G; };
@@ -130,7 +167,7 @@ template <class G> struct Unwrap<void(G)> { using T = G; };
 cudaError_t launchJump32(int mexp, const DevParams32 *params, uint32_t *states,
                          const JumpDesc *descs, int ndesc, int nwords, cudaStream_t s) {
 #define X(M, G) \
-    if (mexp == M) return launch<Tr32, UNWRAP(G)>(params, states, descs, ndesc, nwords, s);
+    if (mexp == M) return launch(UNWRAP(G)(), params, states, descs, ndesc, nwords, s);
     MTGP_JGEO32(X)
 #undef X
     return cudaErrorInvalidValue;
@@ -139,7 +176,7 @@ cudaError_t launchJump32(int mexp, const DevParams32 *params, uint32_t *states,
 cudaError_t launchJump64(int mexp, const DevParams64 *params, uint64_t *states,
                          const JumpDesc *descs, int ndesc, int nwords, cudaStream_t s) {
 #define X(M, G) \
-    if (mexp == M) return launch<Tr64, UNWRAP(G)>(params, states, descs, ndesc, nwords, s);
+    if (mexp == M) return launch(UNWRAP(G)(), params, states, descs, ndesc, nwords, s);
     MTGP_JGEO64(X)
 #undef X
     return cudaErrorInvalidValue;
@@ -150,7 +187,7 @@ cudaError_t launchJumpParts32(int mexp, const DevParams32 *params, const uint32_
                               const JumpPart *parts, int nparts, cudaStream_t s) {
 #define X(M, G)                                                                              \
     if (mexp == M)                                                                          \
-        return launchParts<Tr32, UNWRAP(G)>(params, states, polys, nwords, dst, stride, parts, \
+        return launchParts(UNWRAP(G)(), params, states, polys, nwords, dst, stride, parts, \
                                             nparts, s);
     MTGP_JGEO32(X)
 #undef X
@@ -162,27 +199,11 @@ cudaError_t launchJumpParts64(int mexp, const DevParams64 *params, const uint64_
                               const JumpPart *parts, int nparts, cudaStream_t s) {
 #define X(M, G)                                                                              \
     if (mexp == M)                                                                          \
-        return launchParts<Tr64, UNWRAP(G)>(params, states, polys, nwords, dst, stride, parts, \
+        return launchParts(UNWRAP(G)(), params, states, polys, nwords, dst, stride, parts, \
                                             nparts, s);
     MTGP_JGEO64(X)
 #undef X
     return cudaErrorInvalidValue;
-}
-
-int jumpChunks32(int mexp, int nwords) {
-#define X(M, G) \
-    if (mexp == M) return chunksOf<UNWRAP(G)>(nwords);
-    MTGP_JGEO32(X)
-#undef X
-    return 1;
-}
-
-int jumpChunks64(int mexp, int nwords) {
-#define X(M, G) \
-    if (mexp == M) return chunksOf<UNWRAP(G)>(nwords);
-    MTGP_JGEO64(X)
-#undef X
-    return 1;
 }
 
 namespace {

@@ -198,8 +198,9 @@ int makePlan(Pool<T> &P, const mtgp_work_item_t *items, int nitems, mtgp_gpu_pla
     jparts_b.clear();
     int npre = 0, nmid = 0;
     if (P.tune.jump_parts >= 0 && npolys > 0) {
-        const int tch = T::jumpChunks(P.sh.mexp, (int)pw);
-        const int parts = jumpParts(P.tune, tch);
+        int njumps = 0;
+        for (const BatchTask &t : tasks) njumps += t.j0 >= 0;
+        const int parts = jumpParts(P.tune, njumps, P.pow_width);
         auto addParts = [&](std::vector<JumpPart> &v, uint64_t src, int32_t poly, int32_t dst,
                             int32_t pidx) {
             for (int q = 0; q < parts; q++) {
@@ -208,8 +209,8 @@ int makePlan(Pool<T> &P, const mtgp_work_item_t *items, int nitems, mtgp_gpu_pla
                 d.poly = poly;
                 d.dst = dst;
                 d.pidx = pidx;
-                d.ch0 = (int16_t)partChunk(q, tch, parts);
-                d.ch1 = (int16_t)partChunk(q + 1, tch, parts);
+                d.u0 = (int16_t)partChunk(q, kJumpUnits, parts);
+                d.u1 = (int16_t)partChunk(q + 1, kJumpUnits, parts);
                 v.push_back(d);
             }
         };

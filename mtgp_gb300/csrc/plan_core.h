@@ -33,11 +33,9 @@
 
 namespace mtgp {
 
-// First tap chunk of part q of a jump split into `parts` over `tchunks`
-// chunks (part q covers [partChunk(q), partChunk(q + 1))).  A part generates
-// the sequence up to its last chunk and correlates only its own, so the
-// later parts are the longer ones: the rounding gives the extra chunks to
-// the earlier parts (11 chunks in 4 parts: 3, 3, 3, 2 rather than 2, 3, 3, 3).
+// First unit of part q of a jump split into `parts` over `tchunks` units
+// (part q covers [partChunk(q), partChunk(q + 1))): every unit once, the
+// earlier parts one more where they do not divide evenly.
 inline int partChunk(int q, int tchunks, int parts) {
     const int rem = tchunks % parts;
     return q * (tchunks / parts) + (q < rem ? q : rem);

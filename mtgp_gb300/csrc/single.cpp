@@ -136,8 +136,7 @@ int fillSingle(Obj *h, int kind, void *out, size_t n, void *s) {
     }
     if (!L.d_counter) CK(devMalloc(&L.d_counter, sizeof(unsigned)), "devMalloc(counter)");
     W *win = static_cast<W *>(L.d_win);
-    const int tchunks = T::jumpChunks(P.sh.mexp, pw);
-    const int parts = jumpParts(P.tune, tchunks);
+    const int parts = jumpParts(P.tune, nch - 1, sms);
     const int nparts = (nch - 1) * parts;
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
     const size_t off_items = al(sizeof(BatchTask) * (size_t)nch);
@@ -179,8 +178,8 @@ int fillSingle(Obj *h, int kind, void *out, size_t n, void *s) {
                 d.poly = c - 1;
                 d.dst = c;
                 d.pidx = P.hpidx[0];
-                d.ch0 = (int16_t)partChunk(q, tchunks, parts);
-                d.ch1 = (int16_t)partChunk(q + 1, tchunks, parts);
+                d.u0 = (int16_t)partChunk(q, kJumpUnits, parts);
+                d.u1 = (int16_t)partChunk(q + 1, kJumpUnits, parts);
             }
         CK(cudaMemcpyAsync(L.d_desc, L.h_desc, bytes, cudaMemcpyHostToDevice, S(s)),
            "upload fill descriptors");
