@@ -48,7 +48,8 @@ inline cudaStream_t S(void *s) { return static_cast<cudaStream_t>(s); }
 
 // Tuning knobs (mtgp_gpu_set_tuning).  split_chunk: 0 = automatic, < 0 =
 // never split long requests, > 0 = split into chunks of this many values.
-// batch_grid: 0 = one CTA per resident slot, > 0 = that many CTAs.
+// batch_grid: 0 = automatic (planCtas() CTAs per SM, or every resident slot
+// for the longer exponents), > 0 = that many CTAs.
 // A skip at least this long is done by a GF(2) jump inside the batched
 // kernel (about the work of 2^17 generated values) instead of generation.
 constexpr uint64_t kJumpMinSkip = 1 << 17;
@@ -1146,7 +1147,8 @@ struct mtgp_gpu_plan {
     int ntasks = 0;
     int mode = -2;         // shared output kind of all items, or -2 (mixed)
     uint64_t out_bytes = 0;
-    int grid = 0;
+    int grid = 0;          // CTAs asked for (0 = auto_grid)
+    int auto_grid = 0;     // 0 = every resident slot
     bool split = false;    // some tasks start with an in-kernel jump
     int core = 4;          // 32-bit generation core of unsplit plans
     int64_t chunk = 0;     // chunk length used when splitting

@@ -61,6 +61,15 @@ int makePlan(Pool<T> &P, const mtgp_work_item_t *items, int nitems, mtgp_gpu_pla
     const bool kernel_jumps = T::splits(P.sh.mexp) && (T::kBits == 32 || core == 1);
     // with jumps made ahead of the launch, the kernel without the jump code
     o.resident = o.can_jump ? T::resident(P.sh.mexp, P.tune.jump_parts < 0, core) : 1;
+    // MEXP 11213 and 23209 with jumps made ahead of the launch: few CTAs per
+    // SM and the chunk that goes with them (the longer exponents' CTAs are up
+    // to 1024 threads, and few fit an SM).  A jump costs about mexp^2.
+    const bool few = T::splits(P.sh.mexp) && P.tune.jump_parts >= 0;
+    if (few) {
+        o.sms = P.pow_width;
+        o.ctas = planCtas(P.sh.mexp);
+        o.jump_values = P.sh.mexp == 11213 ? 150 : 1250;
+    }
     // scratch reused by every plan made on this thread
     static thread_local PlanResult R;
     std::string msg;
@@ -265,6 +274,7 @@ int makePlan(Pool<T> &P, const mtgp_work_item_t *items, int nitems, mtgp_gpu_pla
     pl->mode = mode;
     pl->out_bytes = out_bytes;
     pl->grid = (int)P.tune.batch_grid;
+    pl->auto_grid = few ? planCtas(P.sh.mexp) * P.pow_width : 0;
     pl->split = split;
     pl->core = core;
     pl->chunk = cut ? chunk : 0;
@@ -443,7 +453,7 @@ int launchPlan(mtgp_gpu_plan *pl, void *out, void *s) {
     BatchLaunch b{};
     b.mexp = P.sh.mexp;
     b.mode = pl->mode;
-    b.grid = pl->grid;
+    b.grid = pl->grid > 0 ? pl->grid : pl->auto_grid;
     b.nwords = P.polyWords();
     b.polys = pl->d_polys;
     b.split = pl->split;

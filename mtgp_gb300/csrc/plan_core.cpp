@@ -36,6 +36,79 @@ struct Run {
     uint32_t first, n;  // segs of the run in the run-segment array
 };
 
+// How a run of `total` values is cut at chunk length `chunk`: k = ceil(total
+// / chunk) near-equal pieces, rounded up to a multiple of the grain so that
+// the pieces' offsets (and jump polynomials) recur across requests; the last
+// piece takes the rest.  Returns the number of pieces (1: uncut).
+uint64_t cutRun(uint64_t total, uint64_t chunk, uint64_t grain, uint64_t *piece) {
+    *piece = total;
+    if (chunk == 0 || total <= chunk) return 1;
+    const uint64_t k = (total + chunk - 1) / chunk;
+    *piece = ((total + k - 1) / k + grain - 1) / grain * grain;
+    return (total + *piece - 1) / *piece;
+}
+
+// The chunk length with the shortest launch, for o.ctas CTAs per SM, in values
+// generated by one of them (at MEXP 11213 0.59 ns a value on an SM with four,
+// 0.30 with one or two, 32-bit; 1.0 and 0.5 ns 64-bit):
+//   - the jumps, one per piece but a run's first: o.jump_values each (85 and
+//     107 ns on the whole GPU) after the 17 k that the launch before takes;
+//   - the generation: the CTAs' even share of the values, or the long pieces
+//     (over half of the longest) in the rounds that the CTAs need for them,
+//     whichever is longer; the short ones fill what is left.
+// Over 14 workloads (16 to 4096 streams, lognormal and equal lengths, both
+// word sizes) the choice was within 7 % of the best of 15 lengths.  Where no
+// run is longer than jump_min nothing is cut: a pool without jumps needs no
+// jump tables, which take longer to make than such a launch.
+int64_t cheapestChunk(const std::vector<Run> &runs, uint64_t grand, const PlanOptions &o) {
+    constexpr double kJumps = 17000;
+    constexpr uint64_t kShortest = uint64_t(1) << 15;
+    thread_local std::vector<uint64_t> longs;
+    longs.clear();
+    uint64_t longest = 0;
+    for (const Run &R : runs) {
+        if (R.total > kShortest / 2) longs.push_back(R.total);
+        longest = std::max(longest, R.total);
+    }
+    if (longest <= o.jump_min) return (int64_t)o.jump_min;
+    const uint64_t slots = (uint64_t)o.ctas * (uint64_t)o.sms;
+    const double share = (double)grand / (double)slots;
+    int64_t best = 0;
+    double best_cost = 0;
+    // 4, 5, 6 and 7 times a power of two, up to twice the even share or one
+    // that cuts nothing
+    for (uint64_t base = kShortest / 4;; base *= 2) {
+        for (uint64_t m = 4; m < 8; m++) {
+            const uint64_t chunk = m * base, grain = pieceGrain(chunk);
+            uint64_t jumps = 0, top = 0, piece = 0;
+            for (uint64_t t : longs) {
+                jumps += cutRun(t, chunk, grain, &piece) - 1;
+                top = std::max(top, piece);
+            }
+            uint64_t nbig = 0;
+            double big = 0;
+            for (uint64_t t : longs) {
+                const uint64_t k = cutRun(t, chunk, grain, &piece);
+                const uint64_t rest = t - (k - 1) * piece;
+                if (2 * piece > top) nbig += k - 1, big += (double)((k - 1) * piece);
+                if (2 * rest > top) nbig++, big += (double)rest;
+            }
+            const uint64_t tasks = runs.size() + jumps;
+            const uint64_t per_sm = (tasks + (uint64_t)o.sms - 1) / (uint64_t)o.sms;
+            const double slow = std::min(1.0, std::max(0.5, (double)per_sm / o.ctas));
+            const uint64_t rounds = (nbig + slots - 1) / slots;
+            const double gen = std::max(share, rounds <= 1 ? slow * (double)top
+                                                           : (double)rounds * big / (double)nbig);
+            const double cost = gen + (double)o.jump_values * (double)jumps + (jumps ? kJumps : 0);
+            if (!best || cost <= best_cost) {
+                best = (int64_t)chunk;
+                best_cost = cost;
+            }
+            if (jumps == 0 || (double)chunk > 2 * share + (double)o.jump_min) return best;
+        }
+    }
+}
+
 }  // namespace
 
 int planCore(const mtgp_work_item_t *items, int nitems, const PlanOptions &o, PlanResult *r,
@@ -146,6 +219,8 @@ int planCore(const mtgp_work_item_t *items, int nitems, const PlanOptions &o, Pl
     if (o.can_jump) {
         if (o.chunk_tune > 0) {
             chunk = o.chunk_tune;
+        } else if (o.chunk_tune == 0 && o.sms > 0) {
+            chunk = cheapestChunk(runs, grand, o);
         } else if (o.chunk_tune == 0) {
             // a task longer than the average load of one CTA slot would set
             // the length of the whole launch
@@ -164,18 +239,9 @@ int planCore(const mtgp_work_item_t *items, int nitems, const PlanOptions &o, Pl
         const size_t first_task = r->tasks.size();
         for (size_t ri = r0; ri < r1; ri++) {
             const Run &R = runs[ri];
-            // a run longer than one chunk becomes k = ceil(total / chunk)
-            // near-equal pieces, rounded up to a multiple of the grain so
-            // that the pieces' offsets (and jump polynomials) recur across
-            // requests; the last piece takes the rest
-            uint64_t k = 1, piece = R.total;
-            if (chunk > 0 && R.total > (uint64_t)chunk) {
-                k = (R.total + (uint64_t)chunk - 1) / (uint64_t)chunk;
-                piece = (R.total + k - 1) / k;
-                piece = (piece + grain - 1) / grain * grain;
-                k = (R.total + piece - 1) / piece;
-                if (k > 1) cut = true;
-            }
+            uint64_t piece;
+            const uint64_t k = cutRun(R.total, chunk > 0 ? (uint64_t)chunk : 0, grain, &piece);
+            if (k > 1) cut = true;
             uint32_t si = R.first;     // segment of R being cut
             const uint32_t se = R.first + R.n;
             uint64_t used = 0;         // values of it already taken
@@ -212,9 +278,9 @@ int planCore(const mtgp_work_item_t *items, int nitems, const PlanOptions &o, Pl
         if (m > 1) r->stage_streams.push_back(runs[r0].stream);
     }
     r->chunk = cut ? chunk : 0;
-    // longest task first, a jump counted as jump_min generated values (about
-    // its cost)
-    const uint64_t jw = o.can_jump ? o.jump_min : 0;
+    // longest task first, a jump inside the kernel counted as jump_min
+    // generated values (about its cost)
+    const uint64_t jw = o.can_jump && o.sms == 0 ? o.jump_min : 0;
     auto cost = [jw](const PlanTask &t) {
         return t.total + jw * ((t.run ? 1u : 0u) + (t.off ? 1u : 0u));
     };

@@ -49,7 +49,21 @@ struct PlanOptions {
     uint64_t max_gen_skip = uint64_t(1) << 34;
     int64_t chunk_tune = 0;         // > 0 fixed, < 0 never cut, 0 automatic
     int resident = 1;               // resident CTAs of the jumping kernel
+    // > 0: SMs of the GPU, for plans whose jumps are made ahead of the launch
+    // and whose grid is `ctas` CTAs per SM; the automatic chunk is then the
+    // cheapest (cheapestChunk), not a power of two.  jump_values: what a jump
+    // costs, in values generated by one CTA
+    int sms = 0, ctas = 4, jump_values = 150;
 };
+
+// CTAs per SM of a plan's launch, where nothing else is asked for.
+// Four of 11213's fill an SM's data pipe (4096
+// lognormal streams of 32-bit words: 429 us on four, 456 on three and five,
+// 625 on all ten that fit; 1024 streams of 64-bit words: 243 us, 264, 247,
+// 356), and the fewer share it the sooner the longest tasks end, which set
+// the length of a launch.  Two of 23209's, which have twice the threads (512
+// streams: 119 us on two, 144 on three, 168 on four).
+inline int planCtas(int mexp) { return mexp == 11213 ? 4 : 2; }
 
 // One item of a task: count values of kind (-1 = advance without output).
 struct PlanSeg {

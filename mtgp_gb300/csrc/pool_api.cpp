@@ -76,8 +76,8 @@ int autotune(Pool<T> &P, const mtgp_work_item_t *items, int nitems, void *out, v
         return MTGP_OK;
     };
     for (size_t k = 0; k < cands.size() && !rc; k++) {
-        static const int kGridEighths[] = {8, 7, 6, 5, 4};  // of the resident CTAs
-        for (int g = 0; g < 5 && !rc; g++) {
+        static const int kGridEighths[] = {8, 7, 6, 5, 4, 3};  // of the resident CTAs
+        for (int g = 0; g < 6 && !rc; g++) {
             P.tune.split_chunk = cands[k].chunk;
             P.tune.batch_grid = 0;
             P.tune.core = cands[k].core;
@@ -90,13 +90,11 @@ int autotune(Pool<T> &P, const mtgp_work_item_t *items, int nitems, void *out, v
                 delete pl;
                 break;
             }
-            if (g > 0) {
-                // fewer CTAs than resident: fewer share an SM's data pipe,
-                // so each runs its tasks faster, which pays when the longest
-                // tasks set the launch's length
-                const int full = T::resident(P.sh.mexp, pl->split, pl->core);
-                pl->grid = std::max(1, full * kGridEighths[g] / 8);
-            }
+            // fewer CTAs than resident: fewer share an SM's data pipe, so each
+            // runs its tasks faster, which pays when the longest tasks set
+            // the launch's length
+            const int full = T::resident(P.sh.mexp, pl->split, pl->core);
+            pl->grid = std::max(1, full * kGridEighths[g] / 8);
             float ms = 0;
             rc = timeOne(pl, &ms);
             if (rc) {
@@ -107,7 +105,7 @@ int autotune(Pool<T> &P, const mtgp_work_item_t *items, int nitems, void *out, v
             std::snprintf(line, sizeof line, "core=%d chunk=%lld%s grid=%s tasks=%d: %.4f ms\n",
                           pl->core, (long long)pl->chunk,
                           pl->overlap ? " overlap" : "",
-                          g == 0 ? "all" : g == 1 ? "7/8" : g == 2 ? "3/4" : g == 3 ? "5/8" : "1/2",
+                          g == 0 ? "all" : g == 1 ? "7/8" : g == 2 ? "3/4" : g == 3 ? "5/8" : g == 4 ? "1/2" : "3/8",
                           pl->ntasks, ms);
             rep += line;
             if (!*best || ms < best_ms) {
