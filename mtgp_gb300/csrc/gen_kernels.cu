@@ -142,12 +142,20 @@ static cudaError_t gen64x2(int kind, const DevParams64 *params, const int *pidx,
     return cudaGetLastError();
 }
 
+// Values per generator from which the two-word kernels take the long buffer:
+// one and a half of its segments.  Five CTAs an SM still fit, more than its
+// data pipe needs; shorter fills are over before a window moves twice, and
+// keep the ten CTAs of the short one.
+constexpr uint64_t kLongFill = 16384;
+
 template <int N, int TN, int B>
 static cudaError_t gen32_kind(int kind, const DevParams32 *params, const int *pidx,
                               uint32_t *states, int ngen, void *out, uint64_t n,
                               uint64_t os, cudaStream_t s, int core) {
     dim3 grid(ngen), block(TN);
     if (core == 4) return gen32xk<N, TN, B, 4>(kind, params, pidx, states, ngen, out, n, os, s);
+    if (core != 1 && n >= kLongFill)
+        return gen32xk<N, TN, kLongBuf<N, B>, 2>(kind, params, pidx, states, ngen, out, n, os, s);
     if (core != 1) return gen32xk<N, TN, B, 2>(kind, params, pidx, states, ngen, out, n, os, s);
     switch (kind) {
     case -1: k_gen32<N, TN, B, -1><<<grid, block, 0, s>>>(params, pidx, states, out, n, os); break;
@@ -166,6 +174,8 @@ static cudaError_t gen64_kind(int kind, const DevParams64 *params, const int *pi
                               uint64_t *states, int ngen, void *out, uint64_t n,
                               uint64_t os, cudaStream_t s, int core) {
     dim3 grid(ngen), block(TN);
+    if (core != 1 && n >= kLongFill)
+        return gen64x2<N, TN, kLongBuf<N, B>>(kind, params, pidx, states, ngen, out, n, os, s);
     if (core != 1) return gen64x2<N, TN, B>(kind, params, pidx, states, ngen, out, n, os, s);
     switch (kind) {
     case -1: k_gen64<N, TN, B, -1><<<grid, block, 0, s>>>(params, pidx, states, out, n, os); break;

@@ -46,6 +46,13 @@ struct GeoK {
 template <int N, int W, int B>
 using Geo4 = GeoK<N, W, B, 4>;
 
+// The shared buffer (words) of a kernel that runs few CTAs per SM: 45 KB, 42
+// sub-steps before the window moves instead of 14 (the 128 generators: 521 ->
+// 490 us).  The batched kernels keep the short one (412 to 417 us against
+// 416 on 4096 lognormal streams, 449 against 419 on 64-bit words).
+template <int N, int B>
+constexpr int kLongBuf = N == 351 ? 11264 : N == 176 ? 5632 : B;
+
 // Index of sequence position j in the K-plane buffer.
 template <int PW, int K = 4>
 __device__ __forceinline__ int plane_at(int j) {
@@ -80,7 +87,7 @@ struct CoreK {
             int k = threadIdx.x + i * G::T;
             if (k < N) v[i] = buf[plane_at<G::PW, K>(src + k)];
         }
-        __syncthreads();
+        if (src < dst + N) __syncthreads();  // the two overlap
 #pragma unroll
         for (int i = 0; i < PER; i++) {
             int k = threadIdx.x + i * G::T;
@@ -120,32 +127,20 @@ struct CoreK {
         return I;
     }
 
-    // Sub-step k of a segment: K words per thread.  GUARD: the last,
-    // partial sub-step (valid = words of this thread that are inside n).
+    // A sub-step's words and the words that temper them, not yet written out.
+    struct Pend {
+        uint32_t r[K];
+        uint32_t t[K];
+    };
+
+    // The outputs of an earlier sub-step.  GUARD: the last, partial one (valid
+    // = words of this thread inside n).
     template <bool GUARD>
-    __device__ static __forceinline__ void sub(uint32_t *buf, const Idx &I, int k,
-                                               const Lane32 &L, uint32_t mul1, uint32_t otab,
-                                               OT *o, int valid) {
-        const int d = k * G::STEP;
-        uint32_t xs[K + 1], ys[K + 1];
-#pragma unroll
-        for (int c = 0; c <= K; c++) xs[c] = buf[I.x[c] + d];
-#pragma unroll
-        for (int c = 0; c <= K; c++) ys[c] = buf[I.y[c] + d];
-        uint32_t r[K], ov[K];
-#pragma unroll
-        for (int c = 0; c < K; c++) {
-            uint32_t x = (xs[c] & L.mask) ^ xs[c + 1];
-            uint32_t yy = x ^ (x * mul1) ^ (ys[c + 1] >> L.sh2);
-            r[c] = yy ^ lut(L.tbl, yy);
-            if constexpr (KIND >= 0) ov[c] = lut(otab, fold(ys[c]));
-        }
-#pragma unroll
-        for (int c = 0; c < K; c++) buf[I.w[c] + d] = r[c];
+    __device__ static __forceinline__ void emit(const Pend &P, uint32_t otab, OT *o, int valid) {
         if constexpr (KIND >= 0) {
             OT v[K];
 #pragma unroll
-            for (int c = 0; c < K; c++) v[c] = Out32<KIND>::conv(r[c], ov[c]);
+            for (int c = 0; c < K; c++) v[c] = Out32<KIND>::conv(P.r[c], lut(otab, fold(P.t[c])));
             if (!GUARD || valid >= K) {
                 *reinterpret_cast<typename VO::V *>(o) = VO::make(v);
             } else {
@@ -154,6 +149,35 @@ struct CoreK {
                     if (c < valid) o[c] = v[c];
             }
         }
+    }
+
+    // Sub-step k of a segment: K words per thread.  `meanwhile`, the tempering
+    // of the sub-step before, runs between its last shared store and the
+    // barrier: its lookups and stores are then off the chain load - recursion
+    // - store - barrier that one generator's speed hangs on (128 generators of
+    // 2^21 words on a CTA each: 640 us with a sub-step tempered where it is
+    // made, 599 with the tempering after the loads, 521 here; the batched
+    // kernel, whose data pipe is the bound, gains 3 %).
+    template <class F>
+    __device__ static __forceinline__ void sub(uint32_t *buf, const Idx &I, int k, const Lane32 &L,
+                                               uint32_t mul1, Pend &P, F meanwhile) {
+        const int d = k * G::STEP;
+        uint32_t xs[K + 1], ys[K + 1], r[K];
+#pragma unroll
+        for (int c = 0; c <= K; c++) xs[c] = buf[I.x[c] + d];
+#pragma unroll
+        for (int c = 0; c <= K; c++) ys[c] = buf[I.y[c] + d];
+#pragma unroll
+        for (int c = 0; c < K; c++) {
+            uint32_t x = (xs[c] & L.mask) ^ xs[c + 1];
+            const uint32_t yy = x ^ (x * mul1) ^ (ys[c + 1] >> L.sh2);
+            r[c] = yy ^ lut(L.tbl, yy);
+        }
+#pragma unroll
+        for (int c = 0; c < K; c++) buf[I.w[c] + d] = r[c];
+        meanwhile();
+#pragma unroll
+        for (int c = 0; c < K; c++) P.r[c] = r[c], P.t[c] = ys[c];
         __syncthreads();
     }
 
@@ -190,10 +214,14 @@ struct CoreK {
         const Idx I = indices(phase, L.pos);
         OT *o = out + K * t;
         constexpr uint64_t SEG = (uint64_t)G::S * W;
+        Pend P;
         while (n >= SEG) {
 #pragma unroll
             for (int k = 0; k < G::S; k++)
-                sub<false>(buf, I, k, L, mul1, otab, o + k * W, K);
+                sub(buf, I, k, L, mul1, P, [&] {
+                    if (k > 0) emit<false>(P, otab, o + (k - 1) * W, K);
+                });
+            emit<false>(P, otab, o + (G::S - 1) * W, K);
             move(buf, phase + (int)SEG, phase);
             n -= SEG;
             if constexpr (KIND >= 0) o += SEG;
@@ -202,7 +230,10 @@ struct CoreK {
         if (rem > 0) {
             const int subs = (rem + W - 1) / W;
             for (int k = 0; k < subs; k++)
-                sub<true>(buf, I, k, L, mul1, otab, o + k * W, rem - k * W - K * t);
+                sub(buf, I, k, L, mul1, P, [&] {
+                    if (k > 0) emit<false>(P, otab, o + (k - 1) * W, K);
+                });
+            emit<true>(P, otab, o + (subs - 1) * W, rem - (subs - 1) * W - K * t);
         }
         if (phase + rem != 0) move(buf, phase + rem, 0);
     }

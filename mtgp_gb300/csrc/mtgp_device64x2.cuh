@@ -78,7 +78,7 @@ struct Core64x2 {
             int k = threadIdx.x + i * G::T;
             if (k < N) v[i] = buf[at(src + k)];
         }
-        __syncthreads();
+        if (src < dst + N) __syncthreads();  // the two overlap
 #pragma unroll
         for (int i = 0; i < PER; i++) {
             int k = threadIdx.x + i * G::T;
@@ -104,36 +104,53 @@ struct Core64x2 {
         return I;
     }
 
-    // Sub-step k of a segment: two words per thread.  GUARD: the last,
-    // partial sub-step (valid = words of this thread inside n).
+    // A sub-step's words and the words that temper them, not yet written out.
+    struct Pend {
+        uint64_t r[K];
+        uint32_t t[K];
+    };
+
+    // The outputs of an earlier sub-step.  GUARD: the last, partial one (valid
+    // = words of this thread inside n).
     template <bool GUARD>
-    __device__ static __forceinline__ void sub(uint64_t *buf, const Idx &I, int k,
-                                               const Lane64 &L, uint32_t mul1, uint32_t olo,
-                                               uint32_t ohi, OT *o, int valid) {
-        const int d = k * G::STEP;
-        uint64_t xs[K + 1], ys[K + 1];
-#pragma unroll
-        for (int c = 0; c <= K; c++) xs[c] = buf[I.x[c] + d];
-#pragma unroll
-        for (int c = 0; c <= K; c++) ys[c] = buf[I.y[c] + d];
-        uint64_t r[K], ov[K];
-#pragma unroll
-        for (int c = 0; c < K; c++) {
-            r[c] = rec64(xs[c], xs[c + 1], ys[c + 1], L, mul1);
-            if constexpr (KIND >= 0) ov[c] = lut64(olo, ohi, fold((uint32_t)ys[c]));
-        }
-#pragma unroll
-        for (int c = 0; c < K; c++) buf[I.w[c] + d] = r[c];
+    __device__ static __forceinline__ void emit(const Pend &P, uint32_t olo,
+                                                uint32_t ohi, OT *o, int valid) {
         if constexpr (KIND >= 0) {
             OT v[K];
 #pragma unroll
-            for (int c = 0; c < K; c++) v[c] = Out64<KIND>::conv(r[c], ov[c]);
+            for (int c = 0; c < K; c++) v[c] = Out64<KIND>::conv(P.r[c], lut64(olo, ohi, fold(P.t[c])));
             if (!GUARD || valid >= K) {
                 *reinterpret_cast<typename VO::V *>(o) = VO::make(v);
-            } else if (valid > 0) {
-                o[0] = v[0];
+            } else {
+#pragma unroll
+                for (int c = 0; c < K; c++)
+                    if (c < valid) o[c] = v[c];
             }
         }
+    }
+
+    // Sub-step k of a segment: two words per thread.  `meanwhile`, the tempering
+    // of the sub-step before, runs between its loads and their use: off the
+    // chain load - recursion - store - barrier that one generator's speed
+    // hangs on (2^25 values of one generator in 256 chunks: 151 -> 128 us; 144
+    // with the tempering after the stores, as the 32-bit core has it).
+    template <class F>
+    __device__ static __forceinline__ void sub(uint64_t *buf, const Idx &I, int k, const Lane64 &L,
+                                               uint32_t mul1, Pend &P, F meanwhile) {
+        const int d = k * G::STEP;
+        uint64_t xs[K + 1], ys[K + 1];
+#pragma unroll
+        for (int c = 0; c <= K; c++) ys[c] = buf[I.y[c] + d];
+#pragma unroll
+        for (int c = 0; c <= K; c++) xs[c] = buf[I.x[c] + d];
+        meanwhile();
+#pragma unroll
+        for (int c = 0; c < K; c++) {
+            P.r[c] = rec64(xs[c], xs[c + 1], ys[c + 1], L, mul1);
+            P.t[c] = (uint32_t)ys[c];
+        }
+#pragma unroll
+        for (int c = 0; c < K; c++) buf[I.w[c] + d] = P.r[c];
         __syncthreads();
     }
 
@@ -170,10 +187,14 @@ struct Core64x2 {
         const Idx I = indices(phase, L.pos);
         OT *o = out + K * t;
         constexpr uint64_t SEG = (uint64_t)G::S * W;
+        Pend P;
         while (n >= SEG) {
 #pragma unroll
             for (int k = 0; k < G::S; k++)
-                sub<false>(buf, I, k, L, mul1, olo, ohi, o + k * W, K);
+                sub(buf, I, k, L, mul1, P, [&] {
+                    if (k > 0) emit<false>(P, olo, ohi, o + (k - 1) * W, K);
+                });
+            emit<false>(P, olo, ohi, o + (G::S - 1) * W, K);
             move(buf, phase + (int)SEG, phase);
             n -= SEG;
             if constexpr (KIND >= 0) o += SEG;
@@ -182,7 +203,10 @@ struct Core64x2 {
         if (rem > 0) {
             const int subs = (rem + W - 1) / W;
             for (int k = 0; k < subs; k++)
-                sub<true>(buf, I, k, L, mul1, olo, ohi, o + k * W, rem - k * W - K * t);
+                sub(buf, I, k, L, mul1, P, [&] {
+                    if (k > 0) emit<false>(P, olo, ohi, o + (k - 1) * W, K);
+                });
+            emit<true>(P, olo, ohi, o + (subs - 1) * W, rem - (subs - 1) * W - K * t);
         }
         if (phase + rem != 0) move(buf, phase + rem, 0);
     }
