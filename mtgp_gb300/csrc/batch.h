@@ -7,10 +7,10 @@
 namespace mtgp {
 
 struct BatchItem {
-    uint64_t out_off;  // byte offset of the first value in the output buffer
+    uint64_t out_off;  // byte offset of the first value in the output buffer, or its address
     uint64_t count;    // values to produce
     int32_t kind;      // MTGP_KIND_*, or -1 = advance without output
-    int32_t pad_;
+    int32_t direct;    // out_off is an address
 };
 
 struct BatchTask {

@@ -64,6 +64,12 @@ template <> struct SplitGeo32xK<726, 2> { using G = JGeo<726, 23, 256, 256, 4096
 template <int N> constexpr bool kSplit32 = (N == 351 || N == 726);
 template <int N> constexpr bool kSplit64 = (N == 176 || N == 363);
 
+// Where an item's values go.  As an offset from `out` in either case, so that
+// the compiler still sees global memory (generic stores cost 10 %).
+__device__ __forceinline__ char *itemOut(const BatchItem &I, char *out) {
+    return out + (I.out_off - (I.direct ? reinterpret_cast<uintptr_t>(out) : uintptr_t(0)));
+}
+
 // Where a task's start window is: a pre-jumped window, or its stream's.
 template <typename W>
 __device__ __forceinline__ const W *startWindow(const BatchTask &T, const W *states,
@@ -171,7 +177,7 @@ k_batch32(const DevParams32 *__restrict__ params, uint32_t *__restrict__ states,
         __syncthreads();
         for (int i = 0; i < T.nitems; i++) {
             const BatchItem I = items[T.first + i];
-            char *o = out + I.out_off;
+            char *o = itemOut(I, out);
             if constexpr (MODE >= -1) {
                 using OT = typename Out32<(MODE < 0 ? 0 : MODE)>::T;
                 run32<N, TN, B, MODE>(buf, L, L.otab(MODE < 0 ? 0 : MODE), I.count, (OT *)o);
@@ -263,7 +269,7 @@ k_batch32xk(const DevParams32 *__restrict__ params, uint32_t *__restrict__ state
         __syncthreads();
         for (int i = 0; i < TK.nitems; i++) {
             const BatchItem I = items[TK.first + i];
-            char *o = out + I.out_off;
+            char *o = itemOut(I, out);
             if constexpr (MODE >= -1) {
                 using C = CoreK<N, W, B, MODE, K>;
                 C::run(buf, L, L.otab(MODE < 0 ? 0 : MODE), I.count, (typename C::OT *)o);
@@ -322,7 +328,7 @@ k_batch64(const DevParams64 *__restrict__ params, uint64_t *__restrict__ states,
         __syncthreads();
         for (int i = 0; i < T.nitems; i++) {
             const BatchItem I = items[T.first + i];
-            char *o = out + I.out_off;
+            char *o = itemOut(I, out);
             if constexpr (MODE >= -1) {
                 using OT = typename Out64<(MODE < 0 ? 0 : MODE)>::T;
                 run64<N, TN, B, MODE>(buf, L, L.otab_lo(MODE < 0 ? 0 : MODE),
@@ -381,7 +387,7 @@ k_batch64x2(const DevParams64 *__restrict__ params, uint64_t *__restrict__ state
         for (int i = 0; i < TK.nitems; i++) {
             const BatchItem I = items[TK.first + i];
             C::run(buf, L, L.otab_lo(MODE < 0 ? 0 : MODE), L.otab_hi(MODE < 0 ? 0 : MODE),
-                   I.count, (typename C::OT *)(out + I.out_off));
+                   I.count, (typename C::OT *)itemOut(I, out));
         }
         uint64_t *dst = endWindow(TK, states, stage, stateStride(N));
         if (dst)

@@ -1227,7 +1227,7 @@ namespace host {
 // word size.
 template <class T>
 int makePlan(Pool<T> &P, const mtgp_work_item_t *items, int nitems, mtgp_gpu_plan **out,
-             int force_core = 0, int64_t force_chunk = 0);
+             int force_core = 0, int64_t force_chunk = 0, const unsigned char *direct = nullptr);
 template <class T>
 int launchPlan(mtgp_gpu_plan *pl, void *out, void *s);
 int planLaunch(mtgp_gpu_plan *pl, void *out, void *s);

@@ -108,6 +108,11 @@ int recordError(int code, const char *msg);
 // zeroing of new pre-jumped window slots, queued on stream s.  The plan's
 // next launch (or graph capture) then skips them.
 int planPrepare(mtgp_gpu_plan_t *pl, void *s);
+// Make (*pl null) or refill a plan of one pool (the other null) whose items
+// with direct[k] set write at the device address out_offset instead of at that
+// offset of the launch's output buffer.
+int planDirect(mtgp32_gpu_pool_t *p32, mtgp64_gpu_pool_t *p64, const mtgp_work_item_t *items,
+               const unsigned char *direct, int nitems, mtgp_gpu_plan_t **pl);
 void toDev(const mtgp64_params_fast_t &p, DevParams64 *d);
 
 // ---- generation (gen_kernels.cu) ----------------------------------------

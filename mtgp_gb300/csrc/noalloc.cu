@@ -137,7 +137,7 @@ int mtgp32_gpu_batch_noalloc(const mtgp32_params_fast_t *params, int nparams,
         bi.out_off = it.out_offset;
         bi.count = it.count;
         bi.kind = it.kind;
-        bi.pad_ = 0;
+        bi.direct = 0;
         used++;
     }
     for (int st = 0; st < nstreams; st++) {

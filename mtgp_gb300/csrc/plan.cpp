@@ -16,12 +16,13 @@ struct GpuJob {
 
 template <class T>
 int makePlan(Pool<T> &P, const mtgp_work_item_t *items, int nitems, mtgp_gpu_plan **out,
-             int force_core, int64_t force_chunk) {
+             int force_core, int64_t force_chunk, const unsigned char *direct) {
     using W = typename T::W;
     if (!out) return setErr(MTGP_ERR_INVALID, "null plan pointer");
     if (*out && (*out)->pool != &P) return setErr(MTGP_ERR_INVALID, "plan belongs to another pool");
     PlanOptions o;
     o.nstreams = P.count;
+    o.direct = direct;
     o.word_bytes = sizeof(W);
     o.can_jump = planJumps(P);
     o.jump_min = jumpMinSkip(P);
@@ -171,7 +172,7 @@ int makePlan(Pool<T> &P, const mtgp_work_item_t *items, int nitems, mtgp_gpu_pla
         bitems[q].out_off = R.segs[q].out_off;
         bitems[q].count = R.segs[q].count;
         bitems[q].kind = R.segs[q].kind;
-        bitems[q].pad_ = 0;
+        bitems[q].direct = R.segs[q].direct;
     }
     // final indices of the GPU-computed polynomials: after the host's,
     // grouped by parameter set so that each group is one launch
@@ -500,13 +501,19 @@ int planLaunch(mtgp_gpu_plan *pl, void *out, void *s) {
 
 
 template int makePlan<T32>(Pool<T32> &, const mtgp_work_item_t *, int, mtgp_gpu_plan **, int,
-                           int64_t);
+                           int64_t, const unsigned char *);
 template int makePlan<T64>(Pool<T64> &, const mtgp_work_item_t *, int, mtgp_gpu_plan **, int,
-                           int64_t);
+                           int64_t, const unsigned char *);
 template int launchPlan<T32>(mtgp_gpu_plan *, void *, void *);
 template int launchPlan<T64>(mtgp_gpu_plan *, void *, void *);
 
 }  // namespace host
+
+int planDirect(mtgp32_gpu_pool_t *p32, mtgp64_gpu_pool_t *p64, const mtgp_work_item_t *items,
+               const unsigned char *direct, int nitems, mtgp_gpu_plan_t **pl) {
+    return p32 ? makePlan(p32->pool, items, nitems, pl, 0, 0, direct)
+               : makePlan(p64->pool, items, nitems, pl, 0, 0, direct);
+}
 
 int planPrepare(mtgp_gpu_plan_t *pl, void *s) {
     if (!pl) return setErr(MTGP_ERR_INVALID, "null plan");

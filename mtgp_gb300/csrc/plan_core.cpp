@@ -193,22 +193,24 @@ int planCore(const mtgp_work_item_t *items, int nitems, const PlanOptions &o, Pl
                                 "item %d: skip of %llu values would be generated (no in-kernel "
                                 "jump for this exponent); jump the stream instead",
                                 k, (unsigned long long)skip);
-                rseg.push_back(PlanSeg{0, skip, -1});
+                rseg.push_back(PlanSeg{0, skip, -1, 0});
                 cur.n++;
                 cur.total += skip;
                 pos += skip;
             }
             if (count) {
-                rseg.push_back(PlanSeg{it.out_offset, count, it.kind});
+                const bool direct = o.direct && o.direct[k];
+                rseg.push_back(PlanSeg{it.out_offset, count, it.kind, direct});
                 cur.n++;
                 cur.total += count;
                 pos += count;
-                r->out_bytes = std::max(r->out_bytes, it.out_offset + count * o.word_bytes);
+                if (!direct)
+                    r->out_bytes = std::max(r->out_bytes, it.out_offset + count * o.word_bytes);
             }
         }
         if (cur.n || cur.start) {
             if (!cur.n) {  // ends with a jump: a task that only jumps
-                rseg.push_back(PlanSeg{0, 0, -1});
+                rseg.push_back(PlanSeg{0, 0, -1, 0});
                 cur.n = 1;
             }
             grand += cur.total;

@@ -48,6 +48,9 @@ struct PlanOptions {
     uint64_t jump_min = uint64_t(1) << 17;
     uint64_t max_gen_skip = uint64_t(1) << 34;
     int64_t chunk_tune = 0;         // > 0 fixed, < 0 never cut, 0 automatic
+    // per item: its out_offset is a device address, not an offset into the
+    // output buffer (null: none is)
+    const unsigned char *direct = nullptr;
     int resident = 1;               // resident CTAs of the jumping kernel
     // > 0: SMs of the GPU, for plans whose jumps are made ahead of the launch
     // and whose grid is `ctas` CTAs per SM; the automatic chunk is then the
@@ -70,6 +73,7 @@ struct PlanSeg {
     uint64_t out_off;
     uint64_t count;
     int32_t kind;
+    int32_t direct;
 };
 
 struct PlanTask {

@@ -3,8 +3,8 @@
 // The streams of a 32-bit and a 64-bit pool stay resident on the device.
 // Clients submit requests (stream, skip, count, output kind, destination);
 // a scheduler thread admits them into batches and runs each batch as one
-// persistent launch per pool (the batched kernels, through the public plan
-// API):
+// persistent launch per pool (the batched kernels, through plans that are
+// refilled):
 //   - up to `slots` batches are in flight at once, each on its own CUDA
 //     streams (one per pool), so a batch admitted while others run overlaps
 //     them on the GPU, and a batch's two pools run side by side;
@@ -21,8 +21,10 @@
 //     room, else once the batch is planned);
 //   - a request's skip is done by generation when short and by a GF(2) jump
 //     when long (mtgp_work_item_t);
-//   - when a batch completes, results are copied to the callers'
-//     destinations (device or host memory) and its arena block is returned;
+//   - a result whose destination is memory of this device is written there by
+//     the batch's kernel, one for other memory (host, another device) is
+//     copied there from the arena when the batch completes; then its arena
+//     block is returned;
 //     a request without a destination keeps its result in the arena (zero
 //     copy, read through mtgp_server_result) until it is released; the
 //     latency (completion - submission) is recorded.
@@ -150,6 +152,7 @@ struct mtgp_server {
 
     void loop();
     void work(Slot &sl);
+    void markDirect(std::vector<Req> &reqs) const;
     int planBatch(Slot &sl, double *plan_s);
     int launchBatch(Slot &sl);
     int orderBatch(Slot &sl, std::unique_lock<std::mutex> &lk, int rc);
@@ -157,17 +160,89 @@ struct mtgp_server {
     void retireBatch(Slot &sl, int st);
 };
 
-// Refill the slot's plans with the batch (offsets relative to its block).
+// Whether a destination is memory of this device, within one allocation.
+// One batch's look-ups: an allocation is asked for once per batch.
+class DeviceRanges {
+  public:
+    explicit DeviceRanges(int device) : device_(device) {}
+    bool holds(const void *p, uint64_t bytes) {
+        const uint64_t a = reinterpret_cast<uint64_t>(p);
+        for (const auto &r : known_)
+            if (a >= r.first && a - r.first < r.second) return bytes <= r.second - (a - r.first);
+        cudaPointerAttributes at;
+        if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (at.type != cudaMemoryTypeDevice || at.device != device_) return false;
+        unsigned long long base = 0;
+        size_t size = 0;
+        const RangeFn fn = rangeFn();
+        if (!fn || fn(&base, &size, a) != 0 || a < base || a - base >= size) return false;
+        known_.emplace_back(base, size);
+        return bytes <= size - (a - base);
+    }
+
+  private:
+    using RangeFn = int (*)(unsigned long long *, size_t *, unsigned long long);
+    static RangeFn rangeFn() {
+        static const RangeFn fn = [] {
+            void *f = nullptr;
+            cudaDriverEntryPointQueryResult q;
+            if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000,
+                                                 cudaEnableDefault, &q) != cudaSuccess ||
+                q != cudaDriverEntryPointSuccess)
+                f = nullptr;
+            return reinterpret_cast<RangeFn>(f);
+        }();
+        return fn;
+    }
+    int device_;
+    std::vector<std::pair<uint64_t, uint64_t>> known_;  // base, size
+};
+
+// Mark the requests whose values the kernel writes at their destination: in
+// this device's memory, aligned, and apart from every other destination of
+// the batch (those that share memory are copied, in their order, as the last
+// one has to win).  A copy per request bound a burst of 4000 requests with
+// destinations: 11.7 ms of which the kernels are 1.5.
+void mtgp_server::markDirect(std::vector<Req> &reqs) const {
+    struct Span {
+        uint64_t at, end;
+        Req *r;
+    };
+    std::vector<Span> spans;
+    DeviceRanges ranges(device);
+    for (Req &r : reqs) {
+        r.direct = false;
+        if (!r.dst || !r.bytes) continue;
+        const uint64_t at = reinterpret_cast<uint64_t>(r.dst);
+        spans.push_back({at, at + r.bytes, &r});
+        r.direct = at % (r.pool == 0 ? 4 : 8) == 0 && ranges.holds(r.dst, r.bytes);
+    }
+    std::sort(spans.begin(), spans.end(), [](const Span &a, const Span &b) { return a.at < b.at; });
+    size_t top = 0;  // the span that reaches furthest so far
+    for (size_t k = 1; k < spans.size(); k++) {
+        if (spans[k].at < spans[top].end) spans[k].r->direct = spans[top].r->direct = false;
+        if (spans[k].end > spans[top].end) top = k;
+    }
+}
+
+// Refill the slot's plans with the batch (offsets relative to its block, or
+// the destinations themselves).
 int mtgp_server::planBatch(Slot &sl, double *plan_s) {
     std::vector<mtgp_work_item_t> items[2];
+    std::vector<unsigned char> direct[2];
+    markDirect(sl.reqs);
     for (const Req &r : sl.reqs) {
         mtgp_work_item_t it{};
         it.stream = r.stream;
         it.kind = r.kind;
         it.count = r.count;
-        it.out_offset = r.off;
+        it.out_offset = r.direct ? reinterpret_cast<uint64_t>(r.dst) : r.off;
         it.skip = r.skip;
         items[r.pool].push_back(it);
+        direct[r.pool].push_back(r.direct);
     }
     const Clock::time_point tp = Clock::now();
     int rc = MTGP_OK;
@@ -175,13 +250,8 @@ int mtgp_server::planBatch(Slot &sl, double *plan_s) {
         const int n = (int)items[p].size();
         sl.used[p] = n > 0;
         if (!n) continue;
-        if (!sl.plan[p]) {
-            rc = p == 0 ? mtgp32_gpu_pool_plan(p32, items[p].data(), n, &sl.plan[p])
-                        : mtgp64_gpu_pool_plan(p64, items[p].data(), n, &sl.plan[p]);
-        } else {
-            rc = p == 0 ? mtgp32_gpu_pool_replan(p32, items[p].data(), n, sl.plan[p])
-                        : mtgp64_gpu_pool_replan(p64, items[p].data(), n, sl.plan[p]);
-        }
+        rc = mtgp::planDirect(p == 0 ? p32 : nullptr, p == 1 ? p64 : nullptr, items[p].data(),
+                              direct[p].data(), n, &sl.plan[p]);
     }
     *plan_s += std::chrono::duration<double>(Clock::now() - tp).count();
     return rc;
@@ -249,7 +319,7 @@ int mtgp_server::launchBatch(Slot &sl) {
         if (e != cudaSuccess) return mtgp::recordError(MTGP_ERR_CUDA, cudaGetErrorString(e));
     }
     for (const Req &r : sl.reqs) {
-        if (!r.dst || !r.bytes) continue;
+        if (!r.dst || !r.bytes || r.direct) continue;
         e = cudaMemcpyAsync(r.dst, d_arena + r.off, r.bytes, cudaMemcpyDefault, sl.cs[r.pool]);
         if (e != cudaSuccess) return mtgp::recordError(MTGP_ERR_CUDA, cudaGetErrorString(e));
     }

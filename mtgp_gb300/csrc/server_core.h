@@ -74,6 +74,7 @@ struct ServeReq {
     uint64_t skip, count, bytes, off;
     void *dst;
     bool keep;  // no destination: the result stays in the arena until released
+    bool direct;  // the kernel writes at dst
     std::chrono::steady_clock::time_point t_submit;
 };
 
