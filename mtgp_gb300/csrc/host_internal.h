@@ -1138,8 +1138,6 @@ struct mtgp64_gpu {
     Pool<T64> pool;
     SingleFill fill;
 };
-struct mtgp32_gpu_pool { Pool<T32> pool; };
-struct mtgp64_gpu_pool { Pool<T64> pool; };
 
 struct mtgp_gpu_plan {
     int bits = 32;
@@ -1216,6 +1214,48 @@ struct mtgp_gpu_plan {
         cudaFreeHost(h_blob);
         cudaFree(d_counter);
     }
+};
+
+
+// The plan of a pool's latest finished submit, which the next one refills:
+// making its buffers and freeing them took 400 us a call, most of a short
+// one's time.  One plan a pool, none whose buffers grew past kMaxBytes; a
+// submit that finds none (the first, or one of several at once) makes its own.
+class SparePlan {
+  public:
+    ~SparePlan() { delete plan_; }
+    mtgp_gpu_plan *take() {
+        std::lock_guard<std::mutex> lk(mu_);
+        mtgp_gpu_plan *p = plan_;
+        plan_ = nullptr;
+        return p;
+    }
+    // p is idle on the GPU
+    void give(mtgp_gpu_plan *p) {
+        if (!p) return;
+        for (void *b : p->retired_dev) cudaFree(b);
+        for (void *b : p->retired_host) cudaFreeHost(b);
+        p->retired_dev.clear();
+        p->retired_host.clear();
+        if (p->cap_d + p->cap_stage + p->cap_prewin + 4 * p->cap_pscratch <= kMaxBytes) {
+            std::lock_guard<std::mutex> lk(mu_);
+            std::swap(plan_, p);
+        }
+        delete p;
+    }
+
+  private:
+    static constexpr size_t kMaxBytes = size_t(64) << 20;
+    std::mutex mu_;
+    mtgp_gpu_plan *plan_ = nullptr;
+};
+struct mtgp32_gpu_pool {
+    Pool<T32> pool;
+    SparePlan spare;
+};
+struct mtgp64_gpu_pool {
+    Pool<T64> pool;
+    SparePlan spare;
 };
 
 

@@ -253,13 +253,15 @@ extern "C" {
     }                                                                                            \
     int mtgp##B##_gpu_pool_submit(mtgp##B##_gpu_pool_t *p, const mtgp_work_item_t *items,        \
                                   int nitems, void *out, void *s) {                              \
-        mtgp_gpu_plan_t *pl = nullptr;                                                           \
-        int rc = mtgp##B##_gpu_pool_plan(p, items, nitems, &pl);                                 \
-        if (rc) return rc;                                                                       \
-        rc = planLaunch(pl, out, s);                                                             \
-        cudaError_t e = cudaStreamSynchronize(S(s));                                             \
-        delete pl;                                                                               \
-        if (!rc && e != cudaSuccess) rc = cudaErr(e, "batched launch");                          \
+        if (!p) return setErr(MTGP_ERR_INVALID, "null pool");                                    \
+        mtgp_gpu_plan_t *pl = p->spare.take();                                                   \
+        int rc = makePlan(p->pool, items, nitems, &pl);                                          \
+        if (!rc) {                                                                               \
+            rc = planLaunch(pl, out, s);                                                         \
+            const cudaError_t e = cudaStreamSynchronize(S(s));                                   \
+            if (!rc && e != cudaSuccess) rc = cudaErr(e, "batched launch");                      \
+        }                                                                                        \
+        p->spare.give(pl);                                                                       \
         return rc;                                                                               \
     }                                                                                            \
     int mtgp##B##_gpu_pool_jump_polys(mtgp##B##_gpu_pool_t *p, int param_set,                   \
