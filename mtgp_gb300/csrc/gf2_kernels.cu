@@ -25,12 +25,12 @@
 // rows carry zero padding (32 words before, 32 K + 32 after) so that no
 // lane of a visited tile needs a bounds test.  There is no carry-less
 // multiply instruction; a table load stands for WIN shifted XORs.
+#include <cooperative_groups.h>
+
 #include "internal.h"
 
 namespace mtgp {
 namespace {
-
-constexpr int kPowThreads = 1024;
 
 // Output words per lane: K blocks of 32 words (one window extraction serves
 // K table loads); the K x NB accumulators of a lane take 32 registers.  A
@@ -48,20 +48,21 @@ __host__ __device__ constexpr int rowStride(int W) {
     return Comb<WIN>::kPadLo + W + 1 + Comb<WIN>::kPadHi;
 }
 
-// shared words: table (2^WIN rows), R (W), P (2W + 2), Q (W + 1), U (2W + 2)
+// shared words: `tables` tables (2^WIN rows each), R (W), P (2W + 2), Q (W +
+// 1), U (2W + 2)
 template <int WIN>
-__host__ __device__ constexpr size_t powSmemWords(int W) {
-    return (size_t)(1 << WIN) * rowStride<WIN>(W) + (size_t)W + (2 * W + 2) + (W + 1) +
+__host__ __device__ constexpr size_t powSmemWords(int W, int tables) {
+    return (size_t)tables * (1 << WIN) * rowStride<WIN>(W) + (size_t)W + (2 * W + 2) + (W + 1) +
            (2 * W + 2);
 }
 
 // Table rows T[v * S + kPadLo + d] = word d of v * B, d <= lb (B: lb words,
 // generic pointer); the padding stays zero.  Ends with a barrier.
-template <int WIN>
+template <int WIN, int NT>
 __device__ void buildTable(const uint32_t *B, int lb, uint32_t *T, int S) {
     constexpr int R = 1 << WIN;
     const int n = lb + 1;
-    for (int x = threadIdx.x; x < R * n; x += kPowThreads) {
+    for (int x = threadIdx.x; x < R * n; x += NT) {
         const int v = x / n, d = x - v * n;
         const uint32_t hi = d < lb ? B[d] : 0u, lo = d > 0 ? B[d - 1] : 0u;
         uint32_t w = 0;
@@ -83,12 +84,14 @@ __device__ void buildTable(const uint32_t *B, int lb, uint32_t *T, int S) {
 // tiles' A-word pairs are dealt out to the warps in equal contiguous
 // ranges, so that no warp waits for another at the closing barrier; a tile
 // split between warps adds its partial sums with the same atomics.
-template <int WIN>
+// With CS > 1 the pairs are dealt over the warps of CS CTAs, this one the
+// rank-th: Out then holds its share of the sum.
+template <int WIN, int NT, int CS>
 __device__ void combMul(const uint32_t *A, int la, const uint32_t *T, int S, int lb,
-                        uint32_t *Out, int o_lo, int o_hi) {
+                        uint32_t *Out, int o_lo, int o_hi, int rank) {
     constexpr int NB = Comb<WIN>::NB, K = Comb<WIN>::K, IL = Comb<WIN>::IL, PAIRS = IL / 2;
-    constexpr int MASK = (1 << WIN) - 1, nwarps = kPowThreads / 32;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int MASK = (1 << WIN) - 1, nwarps = CS * NT / 32;
+    const int lane = threadIdx.x & 31, warp = rank * (NT / 32) + (threadIdx.x >> 5);
     const int nib = (la + IL - 1) / IL;
     const int ob_lo = (o_lo > 0 ? o_lo - 1 : 0) >> 5;  // o_lo - 1 may carry into o_lo
     const int ob_hi = (o_hi - 1) >> 5;
@@ -168,56 +171,109 @@ __device__ void combMul(const uint32_t *A, int la, const uint32_t *T, int S, int
     __syncthreads();
 }
 
+template <int NT>
 __device__ void zero(uint32_t *p, int n) {
-    for (int w = threadIdx.x; w < n; w += kPowThreads) p[w] = 0;
+    for (int w = threadIdx.x; w < n; w += NT) p[w] = 0;
 }
 
-// R = A * R mod chi (A: generic pointer; R, P, Q, U, T in shared memory).
-template <int WIN>
-__device__ void mulmod(const uint32_t *A, uint32_t *R, const uint32_t *chi, const uint32_t *mu,
-                       int D, int W, uint32_t *T, int S, uint32_t *P, uint32_t *Q, uint32_t *U) {
-    zero(P, 2 * W + 2);
-    buildTable<WIN>(R, W, T, S);
-    combMul<WIN>(A, W, T, S, W, P, 0, 2 * W + 1);  // P = A * R, deg <= 2D - 2
+// The CTAs of a cluster (CS > 1) that share one product: the sum of a word
+// over their copies, and a barrier of all (of the CTA, CS = 1).
+template <int CS>
+struct Team {
+    int rank = 0;
+    __device__ Team() {
+        if constexpr (CS > 1) rank = (int)cooperative_groups::this_cluster().block_rank();
+    }
+    __device__ void sync() const {
+        if constexpr (CS > 1) cooperative_groups::this_cluster().sync();
+        else __syncthreads();
+    }
+    __device__ uint32_t sum(uint32_t *p) const {
+        if constexpr (CS == 1) {
+            return *p;
+        } else {
+            uint32_t v = 0;
+#pragma unroll
+            for (int r = 0; r < CS; r++) v ^= *cooperative_groups::this_cluster().map_shared_rank(p, r);
+            return v;
+        }
+    }
+};
+
+// R = A * R mod chi (A: generic pointer; the others in shared memory).  T:
+// the table of R; Tmu, Tchi: those of mu and chi, or T itself, which are then
+// built where they are needed.  The CTAs of a team all hold R and the tables,
+// and share the pairs of each product.
+template <int WIN, int NT, int CS>
+__device__ void mulmod(const Team<CS> &team, const uint32_t *A, uint32_t *R, const uint32_t *chi,
+                       const uint32_t *mu, int D, int W, uint32_t *T, uint32_t *Tmu,
+                       uint32_t *Tchi, int S, uint32_t *P, uint32_t *Q, uint32_t *U) {
+    zero<NT>(P, 2 * W + 2);
+    zero<NT>(U, 2 * W + 2);
+    buildTable<WIN, NT>(R, W, T, S);
+    // P = A * R, deg <= 2D - 2
+    combMul<WIN, NT, CS>(A, W, T, S, W, P, 0, 2 * W + 1, team.rank);
     const int ws = D >> 5, bs = D & 31;
-    for (int w = threadIdx.x; w < W; w += kPowThreads)  // Q = P >> D
-        Q[w] = __funnelshift_r(P[w + ws], P[w + ws + 1], bs);
-    zero(U, 2 * W + 2);
-    buildTable<WIN>(mu, W, T, S);
-    combMul<WIN>(Q, W, T, S, W, U, ws, 2 * W + 1);  // the words of Q * mu from X^D up
-    for (int w = threadIdx.x; w < W; w += kPowThreads)  // q = (Q * mu) >> D
-        Q[w] = __funnelshift_r(U[w + ws], U[w + ws + 1], bs);
-    buildTable<WIN>(chi, W, T, S);
-    combMul<WIN>(Q, W, T, S, W, P, 0, W);  // P ^= q * chi, below X^W
-    for (int w = threadIdx.x; w < W; w += kPowThreads) {
-        const uint32_t v = P[w];
+    // q >> D of a team's sums: word w from words w + ws and w + ws + 1
+    auto shiftD = [&](uint32_t *from) {
+        for (int w = threadIdx.x; w < W; w += NT)
+            Q[w] = __funnelshift_r(team.sum(from + w + ws), team.sum(from + w + ws + 1), bs);
+    };
+    if constexpr (CS > 1) team.sync();
+    shiftD(P);  // Q = P >> D
+    if (Tmu == T) buildTable<WIN, NT>(mu, W, T, S);
+    else __syncthreads();
+    // the words of Q * mu from X^D up
+    combMul<WIN, NT, CS>(Q, W, Tmu, S, W, U, ws, 2 * W + 1, team.rank);
+    if constexpr (CS > 1) team.sync();  // also: every CTA has read P before it changes below
+    shiftD(U);  // q = (Q * mu) >> D
+    if (Tchi == T) buildTable<WIN, NT>(chi, W, T, S);
+    else __syncthreads();
+    combMul<WIN, NT, CS>(Q, W, Tchi, S, W, P, 0, W, team.rank);  // P ^= q * chi, below X^W
+    if constexpr (CS > 1) team.sync();
+    for (int w = threadIdx.x; w < W; w += NT) {
+        const uint32_t v = team.sum(P + w);
         R[w] = w < ws ? v : w == ws ? (bs ? v & ((1u << bs) - 1u) : 0u) : 0u;
     }
-    __syncthreads();
+    team.sync();  // CS > 1: before any CTA clears its P, or ends
 }
 
-template <int WIN>
-__global__ void __launch_bounds__(kPowThreads, 1)
-k_powops(const PowOp *__restrict__ ops, const uint32_t *__restrict__ scratch, int W) {
+// One step (a product, or a chain of them) per team of CS CTAs.
+//   NT = 1024, CS = 1: one CTA per SM and step.
+//   NT = 512: two CTAs per SM, so that one's tables and barriers run beside
+//     the other's products.
+//   CS = 8: few steps, a cluster each; its time is latency, not bandwidth.
+// keep: the tables of mu and chi have room of their own and are built once.
+template <int WIN, int NT, int CS>
+__global__ void __launch_bounds__(NT, 1024 / NT)
+k_powops(const PowOp *__restrict__ ops, const uint32_t *__restrict__ scratch, int W, int keep) {
     extern __shared__ __align__(16) uint32_t sm[];
+    const Team<CS> team;
     const int S = rowStride<WIN>(W);
-    uint32_t *T = sm, *R = T + (size_t)(1 << WIN) * S, *P = R + W, *Q = P + 2 * W + 2,
-             *U = Q + W + 1;
-    const PowOp &op = ops[blockIdx.x];
-    zero(T, (1 << WIN) * S);  // the rows' padding
+    const size_t TW = (size_t)(1 << WIN) * S;
+    uint32_t *T = sm, *Tmu = T + (keep ? TW : 0), *Tchi = Tmu + (keep ? TW : 0);
+    uint32_t *R = Tchi + TW, *P = R + W, *Q = P + 2 * W + 2, *U = Q + W + 1;
+    const PowOp &op = ops[blockIdx.x / CS];
+    zero<NT>(T, (int)(keep ? 3 * TW : TW));  // the rows' padding
     auto src = [&](int c) -> const uint32_t * {
         return c >= 0 ? op.tab + (size_t)(2 + c) * W : scratch + (size_t)(-1 - c) * W;
     };
     if (op.nsrc == 0) {
-        for (int w = threadIdx.x; w < W; w += kPowThreads) R[w] = w == 0 ? 1u : 0u;
+        for (int w = threadIdx.x; w < W; w += NT) R[w] = w == 0 ? 1u : 0u;
     } else {
         const uint32_t *s0 = src(op.src[0]);
-        for (int w = threadIdx.x; w < W; w += kPowThreads) R[w] = s0[w];
+        for (int w = threadIdx.x; w < W; w += NT) R[w] = s0[w];
     }
     __syncthreads();
+    if (keep && op.nsrc > 1) {
+        buildTable<WIN, NT>(op.tab + W, W, Tmu, S);
+        buildTable<WIN, NT>(op.tab, W, Tchi, S);
+    }
     for (int k = 1; k < op.nsrc; k++)
-        mulmod<WIN>(src(op.src[k]), R, op.tab, op.tab + W, op.D, W, T, S, P, Q, U);
-    for (int w = threadIdx.x; w < W; w += kPowThreads) op.dst[w] = R[w];
+        mulmod<WIN, NT, CS>(team, src(op.src[k]), R, op.tab, op.tab + W, op.D, W, T, Tmu, Tchi, S,
+                            P, Q, U);
+    if (team.rank == 0)
+        for (int w = threadIdx.x; w < W; w += NT) op.dst[w] = R[w];
 }
 
 // Table slot of X^(2^i): 256 m + 2^b for i = 8 m + b (pow_sched.h).
@@ -241,10 +297,12 @@ __global__ void k_gather_pow2(const uint32_t *blk, size_t tw, int W, uint32_t *o
 }
 
 constexpr size_t kPowSmemMax = 200 * 1024;
+constexpr int kPowTeam = 8;  // CTAs that share a step when there are few
+constexpr size_t kPowSmemPair = 113 * 1024;  // two CTAs per SM
 
 }  // namespace
 
-bool powOpsFits(int W) { return W > 0 && powSmemWords<2>(W) * 4 <= kPowSmemMax; }
+bool powOpsFits(int W) { return W > 0 && powSmemWords<2>(W, 1) * 4 <= kPowSmemMax; }
 
 cudaError_t launchMonomials(uint32_t *blk, size_t tw, int W, int n, int i0, cudaStream_t s) {
     if (n <= 0 || i0 <= 0) return cudaSuccess;
@@ -263,15 +321,36 @@ cudaError_t launchPowOps(const PowOp *ops, int n, const uint32_t *scratch, int W
                          cudaStream_t s, int window) {
     if (n <= 0) return cudaSuccess;
     if (!powOpsFits(W)) return cudaErrorInvalidValue;
-    const bool wide = window != 2 && powSmemWords<4>(W) * 4 <= kPowSmemMax;
-    const size_t smem = 4 * (wide ? powSmemWords<4>(W) : powSmemWords<2>(W));
-    auto kern = wide ? k_powops<4> : k_powops<2>;
-    static std::atomic<size_t> seen[2][16];
+    const bool wide = window != 2 && powSmemWords<4>(W, 1) * 4 <= kPowSmemMax;
+    int dev = 0, sms = 152;
+    if (cudaGetDevice(&dev) == cudaSuccess)
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // more steps than SMs: two CTAs per SM (MEXP 11213, whose three tables fit
+    // twice); at most an eighth: a cluster each
+    const bool pairs = wide && n > sms && powSmemWords<4>(W, 3) * 4 <= kPowSmemPair;
+    const bool team = wide && n * kPowTeam <= sms;
+    const bool keep = pairs || (wide && powSmemWords<4>(W, 3) * 4 <= kPowSmemMax);
+    const size_t smem = 4 * (wide ? powSmemWords<4>(W, keep ? 3 : 1) : powSmemWords<2>(W, 1));
+    auto kern = pairs ? k_powops<4, 512, 1>
+              : team  ? k_powops<4, 1024, kPowTeam>
+              : wide  ? k_powops<4, 1024, 1>
+                      : k_powops<2, 1024, 1>;
+    static std::atomic<size_t> seen[4][16];
     cudaError_t e = cudaSuccess;
-    if (smem > 48 * 1024) e = allowSmem(kern, smem, seen[wide]);
+    if (smem > 48 * 1024) e = allowSmem(kern, smem, seen[pairs ? 3 : team ? 2 : wide]);
     if (e != cudaSuccess) return e;
-    kern<<<n, kPowThreads, smem, s>>>(ops, scratch, W);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(team ? n * kPowTeam : n));
+    cfg.blockDim = dim3(pairs ? 512 : 1024);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = kPowTeam;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = team ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, ops, scratch, W, (int)keep);
 }
 
 }  // namespace mtgp
