@@ -25,8 +25,7 @@
 // rows carry zero padding (32 words before, 32 K + 32 after) so that no
 // lane of a visited tile needs a bounds test.  There is no carry-less
 // multiply instruction; a table load stands for WIN shifted XORs.
-#include <cooperative_groups.h>
-
+#include "cta_team.cuh"
 #include "internal.h"
 
 namespace mtgp {
@@ -176,30 +175,6 @@ __device__ void zero(uint32_t *p, int n) {
     for (int w = threadIdx.x; w < n; w += NT) p[w] = 0;
 }
 
-// The CTAs of a cluster (CS > 1) that share one product: the sum of a word
-// over their copies, and a barrier of all (of the CTA, CS = 1).
-template <int CS>
-struct Team {
-    int rank = 0;
-    __device__ Team() {
-        if constexpr (CS > 1) rank = (int)cooperative_groups::this_cluster().block_rank();
-    }
-    __device__ void sync() const {
-        if constexpr (CS > 1) cooperative_groups::this_cluster().sync();
-        else __syncthreads();
-    }
-    __device__ uint32_t sum(uint32_t *p) const {
-        if constexpr (CS == 1) {
-            return *p;
-        } else {
-            uint32_t v = 0;
-#pragma unroll
-            for (int r = 0; r < CS; r++) v ^= *cooperative_groups::this_cluster().map_shared_rank(p, r);
-            return v;
-        }
-    }
-};
-
 // R = A * R mod chi (A: generic pointer; the others in shared memory).  T:
 // the table of R; Tmu, Tchi: those of mu and chi, or T itself, which are then
 // built where they are needed.  The CTAs of a team all hold R and the tables,
@@ -244,17 +219,21 @@ __device__ void mulmod(const Team<CS> &team, const uint32_t *A, uint32_t *R, con
 //     the other's products.
 //   CS = 8: few steps, a cluster each; its time is latency, not bandwidth.
 // keep: the tables of mu and chi have room of their own and are built once.
+// ops null: the steps come as an argument.
 template <int WIN, int NT, int CS>
 __global__ void __launch_bounds__(NT, 1024 / NT)
-k_powops(const PowOp *__restrict__ ops, const uint32_t *__restrict__ scratch, int W, int keep) {
+k_powops(const PowOp *__restrict__ ops, const __grid_constant__ FewOps few,
+         const uint32_t *__restrict__ scratch, int W, int keep) {
     extern __shared__ __align__(16) uint32_t sm[];
     const Team<CS> team;
     const int S = rowStride<WIN>(W);
     const size_t TW = (size_t)(1 << WIN) * S;
     uint32_t *T = sm, *Tmu = T + (keep ? TW : 0), *Tchi = Tmu + (keep ? TW : 0);
     uint32_t *R = Tchi + TW, *P = R + W, *Q = P + 2 * W + 2, *U = Q + W + 1;
-    const PowOp &op = ops[blockIdx.x / CS];
+    __shared__ PowOp op;
+    if (threadIdx.x == 0) op = ops ? ops[blockIdx.x / CS] : few.op[blockIdx.x / CS];
     zero<NT>(T, (int)(keep ? 3 * TW : TW));  // the rows' padding
+    __syncthreads();
     auto src = [&](int c) -> const uint32_t * {
         return c >= 0 ? op.tab + (size_t)(2 + c) * W : scratch + (size_t)(-1 - c) * W;
     };
@@ -317,16 +296,15 @@ cudaError_t launchGatherPow2(const uint32_t *blk, size_t tw, int W, int n, uint3
     return cudaGetLastError();
 }
 
-cudaError_t launchPowOps(const PowOp *ops, int n, const uint32_t *scratch, int W,
-                         cudaStream_t s, int window) {
+static cudaError_t powOps(const PowOp *ops, const FewOps &few, int n, const uint32_t *scratch,
+                          int W, cudaStream_t s, int window) {
     if (n <= 0) return cudaSuccess;
     if (!powOpsFits(W)) return cudaErrorInvalidValue;
     const bool wide = window != 2 && powSmemWords<4>(W, 1) * 4 <= kPowSmemMax;
-    int dev = 0, sms = 152;
-    if (cudaGetDevice(&dev) == cudaSuccess)
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = smCount();
     // more steps than SMs: two CTAs per SM (MEXP 11213, whose three tables fit
-    // twice); at most an eighth: a cluster each
+    // twice; 1000 chains of seven products take 2.01 ms, 2.38 with one CTA);
+    // at most an eighth: a cluster each (one product 56 us -> about 20)
     const bool pairs = wide && n > sms && powSmemWords<4>(W, 3) * 4 <= kPowSmemPair;
     const bool team = wide && n * kPowTeam <= sms;
     const bool keep = pairs || (wide && powSmemWords<4>(W, 3) * 4 <= kPowSmemMax);
@@ -339,18 +317,21 @@ cudaError_t launchPowOps(const PowOp *ops, int n, const uint32_t *scratch, int W
     cudaError_t e = cudaSuccess;
     if (smem > 48 * 1024) e = allowSmem(kern, smem, seen[pairs ? 3 : team ? 2 : wide]);
     if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(team ? n * kPowTeam : n));
-    cfg.blockDim = dim3(pairs ? 512 : 1024);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = kPowTeam;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = team ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, ops, scratch, W, (int)keep);
+    return launchTeams(kern, n, team ? kPowTeam : 1, pairs ? 512 : 1024, smem, s, ops, few,
+                       scratch, W, (int)keep);
+}
+
+cudaError_t launchPowOps(const PowOp *ops, int n, const uint32_t *scratch, int W,
+                         cudaStream_t s, int window) {
+    return powOps(ops, FewOps{}, n, scratch, W, s, window);
+}
+
+cudaError_t launchFewPowOps(const PowOp *host_ops, int n, const uint32_t *scratch, int W,
+                            cudaStream_t s, int window) {
+    if (n > kFewOps) return cudaErrorInvalidValue;
+    FewOps few{};
+    for (int k = 0; k < n; k++) few.op[k] = host_ops[k];
+    return powOps(nullptr, few, n, scratch, W, s, window);
 }
 
 }  // namespace mtgp

@@ -150,6 +150,10 @@ struct T32 {
                             cudaStream_t s) {
         return launchJump32(mexp, p, st, d, nd, nw, s);
     }
+    static cudaError_t jumpRow(int mexp, const DP *p, W *st, const JumpDesc &d, int n, int nw,
+                               cudaStream_t s) {
+        return launchJump32(mexp, p, st, nullptr, n, nw, s, d);
+    }
     static cudaError_t batch(const BatchLaunch &b, const DP *p, W *st, cudaStream_t s) {
         return launchBatch32(b, p, st, s);
     }
@@ -168,9 +172,9 @@ struct T32 {
         return batchResident32(mexp, split, core);
     }
     static bool splits(int mexp) { return batchSplits32(mexp); }
-    static cudaError_t seed(const DP *p, const int *pi, const W *seeds, W *st, int n, int size,
-                            int stride) {
-        return launchSeed32(p, pi, seeds, st, n, size, stride, nullptr);
+    static cudaError_t seed(const DP *p, const int *pi, const W *seeds, W one, W *st, int n,
+                            int size, int stride, cudaStream_t s) {
+        return launchSeed32(p, pi, seeds, one, st, n, size, stride, s);
     }
     static cudaError_t bm(const W *seqs, int n2, int n, int nw, uint32_t *C, int *L) {
         return launchBM32(seqs, n2, n, nw, C, L, nullptr);
@@ -199,6 +203,10 @@ struct T64 {
                             cudaStream_t s) {
         return launchJump64(mexp, p, st, d, nd, nw, s);
     }
+    static cudaError_t jumpRow(int mexp, const DP *p, W *st, const JumpDesc &d, int n, int nw,
+                               cudaStream_t s) {
+        return launchJump64(mexp, p, st, nullptr, n, nw, s, d);
+    }
     static cudaError_t batch(const BatchLaunch &b, const DP *p, W *st, cudaStream_t s) {
         return launchBatch64(b, p, st, s);
     }
@@ -217,9 +225,9 @@ struct T64 {
         return batchResident64(mexp, split, core);
     }
     static bool splits(int mexp) { return batchSplits64(mexp); }
-    static cudaError_t seed(const DP *p, const int *pi, const W *seeds, W *st, int n, int size,
-                            int stride) {
-        return launchSeed64(p, pi, seeds, st, n, size, stride, nullptr);
+    static cudaError_t seed(const DP *p, const int *pi, const W *seeds, W one, W *st, int n,
+                            int size, int stride, cudaStream_t s) {
+        return launchSeed64(p, pi, seeds, one, st, n, size, stride, s);
     }
     static cudaError_t bm(const W *seqs, int n2, int n, int nw, uint32_t *C, int *L) {
         return launchBM64(seqs, n2, n, nw, C, L, nullptr);
@@ -360,7 +368,7 @@ struct Pool {
         cudaError_t e = cudaDeviceSynchronize();
         if (e == cudaSuccess)
             e = cudaMemcpy(d_seeds, seeds, sizeof(W) * count, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = T::seed(d_params, d_pidx, d_seeds, d_states, count, size, stride);
+        if (e == cudaSuccess) e = T::seed(d_params, d_pidx, d_seeds, W(0), d_states, count, size, stride, nullptr);
         if (e == cudaSuccess) e = cudaDeviceSynchronize();
         cudaFree(d_seeds);
         if (e != cudaSuccess) return cudaErr(e, "device seeding");
@@ -921,24 +929,41 @@ struct Pool {
         return MTGP_OK;
     }
 
-    // Jump stream i ahead by `steps` values: X^steps mod chi made on the GPU
-    // (a fraction of a millisecond for any 64-bit distance), then applied.
+    // Jump stream i ahead by `steps` values: X^steps mod chi made on the GPU,
+    // then applied.  Launches only, whose descriptors are their arguments: up
+    // to three levels of products and the jump, in scratch polynomials that
+    // calls on one stream (or ordered with it, as their windows need) use in
+    // turn.  Not for a stream being captured.
     int jumpGpu(int i, uint64_t steps, void *s) {
         if (i < 0 || i >= count) return setErr(MTGP_ERR_INVALID, "stream %d out of range", i);
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        CK(cudaStreamIsCapturing(S(s), &cs), "capture status");
+        if (cs != cudaStreamCaptureStatusNone)
+            return cudaErr(cudaErrorStreamCaptureUnsupported, "jump");
         const int W = polyWords();
-        int rc = ensureScratch((size_t)W, 1);
+        const int k = hpidx[i];
+        const uint32_t *t = nullptr;
+        int rc = gpuPowTables(k, &t);
+        if (!rc) rc = ensureScratch((size_t)(1 + kPowMaxSrc) * W, 1);
         if (rc) return rc;
-        // The scratch buffers are reused: order this call after earlier ones.
-        CK(cudaStreamSynchronize(S(s)), "synchronize");
-        rc = gpuPolys(hpidx[i], &steps, 1, d_poly, s);
-        if (rc) return rc;
+        PowSchedule sch;
+        powSchedule(&steps, 1, powWidth(), sch);
+        std::vector<PowOp> ops;
+        uint32_t *scratch = d_poly + W;  // a tree of eight factors has six inner products
+        powOps(sch, [t](int) { return t; }, d_poly, scratch, chideg[k], ops);
+        size_t first = 0;
+        for (const auto &lev : sch.levels) {
+            CK(launchFewPowOps(ops.data() + first, (int)lev.size(), scratch, W, S(s),
+                               tune.poly_window),
+               "jump polynomial");
+            first += lev.size();
+        }
         JumpDesc d{};
         d.poly[0] = d_poly;
         d.nchain = 1;
-        d.pidx = hpidx[i];
+        d.pidx = k;
         d.src = d.dst = (uint64_t)i * stride;
-        CK(cudaMemcpy(d_desc, &d, sizeof d, cudaMemcpyHostToDevice), "upload descriptor");
-        CK(T::jump(sh.mexp, d_params, d_states, d_desc, 1, W, S(s)), "jump");
+        CK(T::jumpRow(sh.mexp, d_params, d_states, d, 1, W, S(s)), "jump");
         return MTGP_OK;
     }
 
@@ -998,20 +1023,27 @@ struct Pool {
         return jumpArray(i, w.data(), nw, s);
     }
 
-    // Substream j = stream 0's window jumped by j * step (table rows as in
+    // Substream j = the seed's window jumped by j * step (table rows as in
     // cuda-sample/mtgp32-jump-kernel.cuh:383-401: bit b of j applies row
-    // b/2 once for even b, twice for odd b).
-    int substreams(const uint32_t *table, int rows, int nwords, void *s) {
+    // b/2 once for even b, twice for odd b).  A new pool of one parameter set.
+    int substreams(W seed, const uint32_t *table, int rows, int nwords, void *s) {
         if (!table || rows <= 0 || nwords <= 0 || nwords > maxPolyWords())
             return setErr(MTGP_ERR_BAD_JUMP, "bad jump table");
         if (rows < 16 && (uint64_t)count > (1ULL << (2 * rows)))
             return setErr(MTGP_ERR_INVALID, "%d substreams need more than %d table rows", count,
                           rows);
-        int rc = ensureScratch((size_t)rows * nwords, (size_t)count);
+        for (int k = 0; k < 31 && (1 << k) < count; k++)
+            if (k / 2 >= rows)
+                return setErr(MTGP_ERR_INVALID, "%d substreams need more than %d table rows",
+                              count, rows);
+        int rc = ensureScratch((size_t)rows * nwords, 1);
         if (rc) return rc;
-        CK(cudaStreamSynchronize(S(s)), "synchronize");
         CK(cudaMemcpy(d_poly, table, sizeof(uint32_t) * rows * nwords, cudaMemcpyHostToDevice),
            "upload jump table");
+        // the pool's buffers were made and cleared on the default stream, for
+        // which a stream without its ordering does not wait
+        CK(cudaStreamSynchronize(nullptr), "synchronize");
+        CK(T::seed(d_params, d_pidx, nullptr, seed, d_states, 1, size, stride, S(s)), "seed");
         // Doubling: level k makes windows [2^k, 2^(k+1)) from windows
         // [0, 2^k), each by one jump of X^(2^k * step) = table row k/2,
         // applied twice for odd k (the table holds the steps 4^r * step).
@@ -1020,34 +1052,19 @@ struct Pool {
         // row b/2 once or twice, lowest bit first) in the same order, so the
         // windows are bit-identical to it, with one jump per substream
         // instead of up to 2 * rows; the levels run one launch each.
-        std::vector<JumpDesc> descs;
-        descs.reserve(count);
-        std::vector<int> level_end;
         for (int k = 0; k < 31 && (1 << k) < count; k++) {
-            if (k / 2 >= rows)
-                return setErr(MTGP_ERR_INVALID, "%d substreams need more than %d table rows",
-                              count, rows);
-            const uint32_t *row = d_poly + (size_t)(k / 2) * nwords;
-            for (int j = 0; j < (1 << k) && j + (1 << k) < count; j++) {
-                JumpDesc d{};
-                d.poly[d.nchain++] = row;
-                if (k & 1) d.poly[d.nchain++] = row;
-                d.pidx = hpidx[j];
-                d.src = (uint64_t)j * stride;
-                d.dst = (uint64_t)(j + (1 << k)) * stride;
-                descs.push_back(d);
+            JumpDesc d{};
+            d.poly[d.nchain++] = d_poly + (size_t)(k / 2) * nwords;
+            if (k & 1) {
+                d.poly[1] = d.poly[0];
+                d.nchain++;
             }
-            level_end.push_back((int)descs.size());
-        }
-        if (descs.empty()) return MTGP_OK;
-        CK(cudaMemcpy(d_desc, descs.data(), sizeof(JumpDesc) * descs.size(),
-                      cudaMemcpyHostToDevice),
-           "upload descriptors");
-        int first = 0;
-        for (int end : level_end) {
-            CK(T::jump(sh.mexp, d_params, d_states, d_desc + first, end - first, nwords, S(s)),
+            d.pidx = hpidx[0];
+            d.dst = (uint64_t)(1 << k) * stride;
+            d.step = (uint64_t)stride;
+            CK(T::jumpRow(sh.mexp, d_params, d_states, d, std::min(1 << k, count - (1 << k)),
+                          nwords, S(s)),
                "jump");
-            first = end;
         }
         return MTGP_OK;
     }

@@ -120,10 +120,11 @@ void toDev(const mtgp64_params_fast_t &p, DevParams64 *d);
 // arrays), its window at states + g*stateStride(N), and writes n values of
 // `kind` at out + g*outStride elements.  kind < 0 = skip (no output).
 // Integer seeding of `count` windows (size words each, `stride` apart) on
-// the device: stream i from seeds[i] with parameter set pidx[i].
-cudaError_t launchSeed32(const DevParams32 *params, const int *pidx, const uint32_t *seeds,
+// the device: stream i from seeds[i] (or all from `one`, seeds null) with
+// parameter set pidx[i].
+cudaError_t launchSeed32(const DevParams32 *params, const int *pidx, const uint32_t *seeds, uint32_t one,
                          uint32_t *states, int count, int size, int stride, cudaStream_t s);
-cudaError_t launchSeed64(const DevParams64 *params, const int *pidx, const uint64_t *seeds,
+cudaError_t launchSeed64(const DevParams64 *params, const int *pidx, const uint64_t *seeds, uint64_t one,
                          uint64_t *states, int count, int size, int stride, cudaStream_t s);
 // Key-schedule seeding (init_by_array / init_by_str) on the device: stream
 // i from the key words keys[koff[i] .. koff[i+1]).
@@ -171,6 +172,14 @@ cudaError_t launchGatherPow2(const uint32_t *blk, size_t tw, int W, int n, uint3
 // table fits in shared memory, else 2), 2 or 4.
 cudaError_t launchPowOps(const PowOp *ops, int n, const uint32_t *scratch, int W,
                          cudaStream_t s, int window = 0);
+// The same for at most kFewOps steps given by the host: a kernel argument, no
+// upload.
+constexpr int kFewOps = 8;
+struct FewOps {
+    PowOp op[kFewOps];
+};
+cudaError_t launchFewPowOps(const PowOp *host_ops, int n, const uint32_t *scratch, int W,
+                            cudaStream_t s, int window = 0);
 
 // core: the 32-bit generation core, 2 = two adjacent words per thread (the
 // default), 4 = four, 1 = one word per thread.
@@ -197,6 +206,7 @@ struct JumpDesc {
     int pidx;          // parameter-set index
     uint64_t src;      // element offset of the source window
     uint64_t dst;      // element offset of the destination window
+    uint64_t step;     // of a row of jumps: offset from one's windows to the next's
 };
 // Partial jumps: CTA b correlates the share [u0, u1) of kJumpUnits of one
 // jump's taps and XORs the result into its destination window (zero on
@@ -224,11 +234,13 @@ cudaError_t launchChunkWindows32(const uint32_t *gen, uint32_t *win, int n, int 
                                  cudaStream_t s);
 cudaError_t launchChunkWindows64(const uint64_t *gen, uint64_t *win, int n, int stride, int nwin,
                                  cudaStream_t s);
+// descs null: a row of jumps by the same polynomials, described by `row` (a
+// kernel argument, no upload).
 cudaError_t launchJump32(int mexp, const DevParams32 *params, uint32_t *states,
                          const JumpDesc *descs, int ndesc, int nwords,
-                         cudaStream_t s);
+                         cudaStream_t s, const JumpDesc &row = JumpDesc{});
 cudaError_t launchJump64(int mexp, const DevParams64 *params, uint64_t *states,
                          const JumpDesc *descs, int ndesc, int nwords,
-                         cudaStream_t s);
+                         cudaStream_t s, const JumpDesc &row = JumpDesc{});
 
 }  // namespace mtgp

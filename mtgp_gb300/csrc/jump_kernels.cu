@@ -1,33 +1,43 @@
-// jump_kernels.cu -- jump-ahead of many windows, one CTA per descriptor.
+// jump_kernels.cu -- jump-ahead of many windows, one team of CTAs per
+// descriptor.
 //
 // Each descriptor names a source window, a destination window and a chain
 // of polynomials (jump_sorted.cuh).  Substream j of the reference's CUDA
 // sample is reached the same way, from the table of X^(4^k * 3^162) mod chi
 // (cuda-sample/mtgp32-jump-kernel.cuh:383-401), but there one thread steps
 // the recursion for every coefficient; here the whole CTA does.
+#include "cta_team.cuh"
 #include "jump_sorted.cuh"
 
 namespace mtgp {
 
 namespace {
 
-template <class G>
+// A team of CS CTAs per descriptor, each with its share of every polynomial's
+// patterns; all make the sequence, which takes them as long as one.
+template <class G, int CS>
 __global__ void __launch_bounds__(G::NT, G::MINB)
 k_jump(const typename G::Tr::P *__restrict__ params, typename G::W *__restrict__ states,
-       const JumpDesc *__restrict__ descs, int nwords) {
+       const JumpDesc *__restrict__ descs, const __grid_constant__ JumpDesc row, int nwords) {
     using W = typename G::W;
     extern __shared__ __align__(16) unsigned char smem[];
+    const Team<CS> team;
     W *seq = reinterpret_cast<W *>(smem);
-    const W *jout = reinterpret_cast<const W *>(smem + G::off_jout);
-    const JumpDesc &D = descs[blockIdx.x];
+    W *jout = reinterpret_cast<W *>(smem + G::off_jout);
+    const JumpDesc &D = descs ? descs[blockIdx.x / CS] : row;
+    const uint64_t at = descs ? 0 : blockIdx.x / CS * row.step;
     typename G::Tr::Lane L;
     L.load(params[D.pidx], threadIdx.x & 31);
-    for (int k = threadIdx.x; k < G::N; k += G::NT) seq[k] = states[D.src + k];
+    for (int k = threadIdx.x; k < G::N; k += G::NT) seq[k] = states[D.src + at + k];
     for (int c = 0; c < D.nchain; c++) {
-        jumpSorted<G>(smem, L, D.poly[c], nwords, 0, kJumpUnits);
-        for (int k = threadIdx.x; k < G::N; k += G::NT) seq[k] = jout[k];
+        jumpSorted<G>(smem, L, D.poly[c], nwords, kJumpUnits * team.rank / CS,
+                      kJumpUnits * (team.rank + 1) / CS);
+        if constexpr (CS > 1) team.sync();
+        for (int k = threadIdx.x; k < G::N; k += G::NT) seq[k] = team.sum(jout + k);
+        if constexpr (CS > 1) team.sync();  // before any CTA clears its share, or ends
     }
-    for (int k = threadIdx.x; k < G::N; k += G::NT) states[D.dst + k] = seq[k];
+    if (team.rank == 0)
+        for (int k = threadIdx.x; k < G::N; k += G::NT) states[D.dst + at + k] = seq[k];
 }
 
 // One CTA per (jump, share of its rows): XOR-ed into the zeroed destination
@@ -57,16 +67,17 @@ k_jump_part(const typename G::Tr::P *__restrict__ params, const typename G::W *_
 template <class Tr, class Geo>
 __global__ void __launch_bounds__(Geo::NT)
 k_jump_ring(const typename Tr::P *__restrict__ params, typename Tr::W *__restrict__ states,
-            const JumpDesc *__restrict__ descs, int nwords) {
+            const JumpDesc *__restrict__ descs, const __grid_constant__ JumpDesc row, int nwords) {
     using W = typename Tr::W;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     W *smem = reinterpret_cast<W *>(smem_raw);
-    const JumpDesc &D = descs[blockIdx.x];
+    const JumpDesc &D = descs ? descs[blockIdx.x] : row;
+    const uint64_t at = descs ? 0 : blockIdx.x * row.step;
     typename Tr::Lane L;
     L.load(params[D.pidx], threadIdx.x & 31);
-    for (int k = threadIdx.x; k < Geo::N; k += Geo::NT) smem[k] = states[D.src + k];
+    for (int k = threadIdx.x; k < Geo::N; k += Geo::NT) smem[k] = states[D.src + at + k];
     jump_chain<Tr, Geo>(smem, L, D.poly, D.nchain, nwords);
-    for (int k = threadIdx.x; k < Geo::N; k += Geo::NT) states[D.dst + k] = smem[k];
+    for (int k = threadIdx.x; k < Geo::N; k += Geo::NT) states[D.dst + at + k] = smem[k];
 }
 
 // A share [u0, u1) of kJumpUnits here is a range of whole chunks of taps.
@@ -109,13 +120,14 @@ cudaError_t launchParts(Ring<Tr, Geo>, const typename Tr::P *params, const typen
 
 template <class Tr, class Geo>
 cudaError_t launch(Ring<Tr, Geo>, const typename Tr::P *params, typename Tr::W *states,
-                   const JumpDesc *descs, int ndesc, int nwords, cudaStream_t s) {
+                   const JumpDesc *descs, int ndesc, int nwords, cudaStream_t s,
+                   const JumpDesc &row) {
     const size_t smem = Geo::template bytes<typename Tr::W>(nwords);
     static std::atomic<size_t> seen[16];
     cudaError_t e = allowSmem(k_jump_ring<Tr, Geo>, smem, seen);
     if (e != cudaSuccess) return e;
     if (ndesc <= 0) return cudaSuccess;
-    k_jump_ring<Tr, Geo><<<ndesc, Geo::NT, smem, s>>>(params, states, descs, nwords);
+    k_jump_ring<Tr, Geo><<<ndesc, Geo::NT, smem, s>>>(params, states, descs, row, nwords);
     return cudaGetLastError();
 }
 
@@ -132,15 +144,27 @@ cudaError_t launchParts(G, const typename G::Tr::P *params, const typename G::W 
     return cudaGetLastError();
 }
 
+template <class G, int CS>
+cudaError_t launchTeam(const typename G::Tr::P *params, typename G::W *states,
+                       const JumpDesc *descs, int ndesc, int nwords, cudaStream_t s,
+                       const JumpDesc &row) {
+    static std::atomic<size_t> seen[16];
+    cudaError_t e = allowSmem(k_jump<G, CS>, G::kBytes, seen);
+    if (e != cudaSuccess) return e;
+    return launchTeams(k_jump<G, CS>, ndesc, CS, G::NT, G::kBytes, s, params, states, descs, row,
+                       nwords);
+}
+
+// CTAs per jump: as many as leave one per SM at most.
 template <class G>
 cudaError_t launch(G, const typename G::Tr::P *params, typename G::W *states, const JumpDesc *descs,
-                   int ndesc, int nwords, cudaStream_t s) {
-    static std::atomic<size_t> seen[16];
-    cudaError_t e = allowSmem(k_jump<G>, G::kBytes, seen);
-    if (e != cudaSuccess) return e;
+                   int ndesc, int nwords, cudaStream_t s, const JumpDesc &row) {
     if (ndesc <= 0) return cudaSuccess;
-    k_jump<G><<<ndesc, G::NT, G::kBytes, s>>>(params, states, descs, nwords);
-    return cudaGetLastError();
+    const int sms = smCount();
+    if (8 * ndesc <= sms) return launchTeam<G, 8>(params, states, descs, ndesc, nwords, s, row);
+    if (4 * ndesc <= sms) return launchTeam<G, 4>(params, states, descs, ndesc, nwords, s, row);
+    if (2 * ndesc <= sms) return launchTeam<G, 2>(params, states, descs, ndesc, nwords, s, row);
+    return launchTeam<G, 1>(params, states, descs, ndesc, nwords, s, row);
 }
 
 }  // namespace
@@ -165,18 +189,20 @@ template <class G> struct Unwrap<void(G)> { using T = G; };
 #define UNWRAP(G) typename Unwrap<void G>::T
 
 cudaError_t launchJump32(int mexp, const DevParams32 *params, uint32_t *states,
-                         const JumpDesc *descs, int ndesc, int nwords, cudaStream_t s) {
+                         const JumpDesc *descs, int ndesc, int nwords, cudaStream_t s,
+                         const JumpDesc &row) {
 #define X(M, G) \
-    if (mexp == M) return launch(UNWRAP(G)(), params, states, descs, ndesc, nwords, s);
+    if (mexp == M) return launch(UNWRAP(G)(), params, states, descs, ndesc, nwords, s, row);
     MTGP_JGEO32(X)
 #undef X
     return cudaErrorInvalidValue;
 }
 
 cudaError_t launchJump64(int mexp, const DevParams64 *params, uint64_t *states,
-                         const JumpDesc *descs, int ndesc, int nwords, cudaStream_t s) {
+                         const JumpDesc *descs, int ndesc, int nwords, cudaStream_t s,
+                         const JumpDesc &row) {
 #define X(M, G) \
-    if (mexp == M) return launch(UNWRAP(G)(), params, states, descs, ndesc, nwords, s);
+    if (mexp == M) return launch(UNWRAP(G)(), params, states, descs, ndesc, nwords, s, row);
     MTGP_JGEO64(X)
 #undef X
     return cudaErrorInvalidValue;

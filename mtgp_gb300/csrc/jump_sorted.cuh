@@ -68,10 +68,10 @@ struct SJump {
     static_assert(kBytes <= 227 * 1024, "jump buffers exceed shared memory");
 };
 
-// Barrier `id` of `threads` threads.  The form that does not need a warp to
-// arrive together: the loops before it end at different trips within a warp.
+// Barrier `id` of `threads` threads, whole warps.
 __device__ __forceinline__ void barN(int id, int threads) {
-    asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+    __syncwarp();  // the loops before it end at different trips within a warp
+    asm volatile("barrier.sync.aligned %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
 // Rank of pattern p in Gray-code order (p = rank ^ rank >> 1).

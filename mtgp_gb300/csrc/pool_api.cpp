@@ -210,11 +210,7 @@ extern "C" {
                                              int nwords, void *s) {                              \
         int rc = newObj(out);                                                                    \
         if (!rc) rc = (*out)->pool.init(p, 1, nullptr, count);                                   \
-        if (!rc) {                                                                               \
-            std::vector<W> seeds((size_t)count, seed);                                           \
-            rc = (*out)->pool.seedAll(seeds.data());                                             \
-        }                                                                                        \
-        if (!rc) rc = (*out)->pool.substreams(table, rows, nwords, s);                           \
+        if (!rc) rc = (*out)->pool.substreams(seed, table, rows, nwords, s);                     \
         if (rc && out && *out) {                                                                 \
             delete *out;                                                                         \
             *out = nullptr;                                                                      \
