@@ -33,6 +33,14 @@ struct Team {
     }
 };
 
+// CTAs per team for n teams at once: as many as leave one per SM, with a
+// quarter of the SMs to spare, as a cluster needs its SMs close together (16
+// teams of eight no longer run side by side).
+inline int teamSize(int n, int sms) {
+    const int room = sms - sms / 4;
+    return 8 * n <= room ? 8 : 4 * n <= room ? 4 : 2 * n <= room ? 2 : 1;
+}
+
 // Launch `kern` on n teams of `cs` CTAs.
 template <class K, class... Args>
 cudaError_t launchTeams(K kern, int n, int cs, int threads, size_t smem, cudaStream_t s,

@@ -217,7 +217,7 @@ __device__ void mulmod(const Team<CS> &team, const uint32_t *A, uint32_t *R, con
 //   NT = 1024, CS = 1: one CTA per SM and step.
 //   NT = 512: two CTAs per SM, so that one's tables and barriers run beside
 //     the other's products.
-//   CS = 8: few steps, a cluster each; its time is latency, not bandwidth.
+//   CS > 1: few steps, a cluster each; their time is latency, not bandwidth.
 // keep: the tables of mu and chi have room of their own and are built once.
 // ops null: the steps come as an argument.
 template <int WIN, int NT, int CS>
@@ -276,7 +276,6 @@ __global__ void k_gather_pow2(const uint32_t *blk, size_t tw, int W, uint32_t *o
 }
 
 constexpr size_t kPowSmemMax = 200 * 1024;
-constexpr int kPowTeam = 8;  // CTAs that share a step when there are few
 constexpr size_t kPowSmemPair = 113 * 1024;  // two CTAs per SM
 
 }  // namespace
@@ -304,20 +303,22 @@ static cudaError_t powOps(const PowOp *ops, const FewOps &few, int n, const uint
     const int sms = smCount();
     // more steps than SMs: two CTAs per SM (MEXP 11213, whose three tables fit
     // twice; 1000 chains of seven products take 2.01 ms, 2.38 with one CTA);
-    // at most an eighth: a cluster each (one product 56 us -> about 20)
+    // few: a cluster each (one product 56 -> 31 us)
     const bool pairs = wide && n > sms && powSmemWords<4>(W, 3) * 4 <= kPowSmemPair;
-    const bool team = wide && n * kPowTeam <= sms;
+    const int team = wide ? teamSize(n, sms) : 1;
     const bool keep = pairs || (wide && powSmemWords<4>(W, 3) * 4 <= kPowSmemMax);
     const size_t smem = 4 * (wide ? powSmemWords<4>(W, keep ? 3 : 1) : powSmemWords<2>(W, 1));
     auto kern = pairs ? k_powops<4, 512, 1>
-              : team  ? k_powops<4, 1024, kPowTeam>
-              : wide  ? k_powops<4, 1024, 1>
-                      : k_powops<2, 1024, 1>;
-    static std::atomic<size_t> seen[4][16];
+              : team == 8 ? k_powops<4, 1024, 8>
+              : team == 4 ? k_powops<4, 1024, 4>
+              : team == 2 ? k_powops<4, 1024, 2>
+              : wide      ? k_powops<4, 1024, 1>
+                          : k_powops<2, 1024, 1>;
+    static std::atomic<size_t> seen[10][16];
     cudaError_t e = cudaSuccess;
-    if (smem > 48 * 1024) e = allowSmem(kern, smem, seen[pairs ? 3 : team ? 2 : wide]);
+    if (smem > 48 * 1024) e = allowSmem(kern, smem, seen[pairs ? 9 : wide ? team : 0]);
     if (e != cudaSuccess) return e;
-    return launchTeams(kern, n, team ? kPowTeam : 1, pairs ? 512 : 1024, smem, s, ops, few,
+    return launchTeams(kern, n, team, pairs ? 512 : 1024, smem, s, ops, few,
                        scratch, W, (int)keep);
 }
 

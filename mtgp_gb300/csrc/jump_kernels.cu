@@ -155,16 +155,16 @@ cudaError_t launchTeam(const typename G::Tr::P *params, typename G::W *states,
                        nwords);
 }
 
-// CTAs per jump: as many as leave one per SM at most.
 template <class G>
 cudaError_t launch(G, const typename G::Tr::P *params, typename G::W *states, const JumpDesc *descs,
                    int ndesc, int nwords, cudaStream_t s, const JumpDesc &row) {
     if (ndesc <= 0) return cudaSuccess;
-    const int sms = smCount();
-    if (8 * ndesc <= sms) return launchTeam<G, 8>(params, states, descs, ndesc, nwords, s, row);
-    if (4 * ndesc <= sms) return launchTeam<G, 4>(params, states, descs, ndesc, nwords, s, row);
-    if (2 * ndesc <= sms) return launchTeam<G, 2>(params, states, descs, ndesc, nwords, s, row);
-    return launchTeam<G, 1>(params, states, descs, ndesc, nwords, s, row);
+    switch (teamSize(ndesc, smCount())) {
+    case 8: return launchTeam<G, 8>(params, states, descs, ndesc, nwords, s, row);
+    case 4: return launchTeam<G, 4>(params, states, descs, ndesc, nwords, s, row);
+    case 2: return launchTeam<G, 2>(params, states, descs, ndesc, nwords, s, row);
+    default: return launchTeam<G, 1>(params, states, descs, ndesc, nwords, s, row);
+    }
 }
 
 }  // namespace

@@ -29,6 +29,12 @@ uint64_t pieceGrain(uint64_t chunk) {
     return g;
 }
 
+// The grain of plans whose chunk is the cheapest: 2^16, or 2^15 below chunks of
+// 2^19.  The offsets are then multiples of it up to a run's length, few for a
+// whole plan, and those of 2^16 are table polynomials: a plan's first launch
+// makes no products for them.
+uint64_t cheapGrain(uint64_t chunk) { return uint64_t(1) << (chunk >= uint64_t(1) << 19 ? 16 : 15); }
+
 // A run: consecutive generated work of one stream starting at `start`.
 struct Run {
     int32_t stream;
@@ -50,7 +56,8 @@ uint64_t cutRun(uint64_t total, uint64_t chunk, uint64_t grain, uint64_t *piece)
 
 // The chunk length with the shortest launch, for o.ctas CTAs per SM, in values
 // generated by one of them (at MEXP 11213 0.59 ns a value on an SM with four,
-// 0.30 with one or two, 32-bit; 1.0 and 0.5 ns 64-bit):
+// 0.42 with three, 0.30 with one or two, 32-bit; 1.0 ns with three or four and
+// 0.75 with fewer, 64-bit):
 //   - the jumps, one per piece but a run's first: o.jump_values each (85 and
 //     107 ns on the whole GPU) after the 17 k that the launch before takes;
 //   - the generation: the CTAs' even share of the values, or the long pieces
@@ -79,7 +86,7 @@ int64_t cheapestChunk(const std::vector<Run> &runs, uint64_t grand, const PlanOp
     // that cuts nothing
     for (uint64_t base = kShortest / 4;; base *= 2) {
         for (uint64_t m = 4; m < 8; m++) {
-            const uint64_t chunk = m * base, grain = pieceGrain(chunk);
+            const uint64_t chunk = m * base, grain = cheapGrain(chunk);
             uint64_t jumps = 0, top = 0, piece = 0;
             for (uint64_t t : longs) {
                 jumps += cutRun(t, chunk, grain, &piece) - 1;
@@ -95,7 +102,8 @@ int64_t cheapestChunk(const std::vector<Run> &runs, uint64_t grand, const PlanOp
             }
             const uint64_t tasks = runs.size() + jumps;
             const uint64_t per_sm = (tasks + (uint64_t)o.sms - 1) / (uint64_t)o.sms;
-            const double slow = std::min(1.0, std::max(0.5, (double)per_sm / o.ctas));
+            const double slow = std::min(1.0, o.word_bytes == 4 ? std::max(0.5, (double)per_sm / o.ctas)
+                                              : 2 * per_sm <= (uint64_t)o.ctas ? 0.75 : 1.0);
             const uint64_t rounds = (nbig + slots - 1) / slots;
             const double gen = std::max(share, rounds <= 1 ? slow * (double)top
                                                            : (double)rounds * big / (double)nbig);
@@ -232,7 +240,10 @@ int planCore(const mtgp_work_item_t *items, int nitems, const PlanOptions &o, Pl
         }
     }
     // cut runs into tasks; per stream, mark write-back
-    const uint64_t grain = chunk > 0 ? pieceGrain((uint64_t)chunk) : 1;
+    const bool cheap = o.sms > 0 && o.chunk_tune == 0;
+    const uint64_t grain = chunk <= 0 ? 1
+                           : cheap   ? cheapGrain((uint64_t)chunk)
+                                     : pieceGrain((uint64_t)chunk);
     r->segs.reserve(rseg.size() + runs.size());
     bool cut = false;
     for (size_t r0 = 0, r1; r0 < runs.size(); r0 = r1) {
