@@ -439,7 +439,8 @@ int mtgp_gpu_plan_describe(const mtgp_gpu_plan_t *plan, int64_t *values,
  *   "jump_parts"   jumps made ahead of a batched launch (the chunk starts of
  *                  such a fill, and batched tasks that start with a jump):
  *                  CTAs per jump, 0 = automatic (1 to 8, by the number of
- *                  jumps), > 0 = that many (at most 32); -1 = such jumps run
+ *                  jumps), > 0 = that many (at most 32; in a fill the next
+ *                  lower power of two, at most 8); -1 = such jumps run
  *                  inside the batched kernel instead
  *   "jump_overlap" 0 = the jump parts run before the persistent launch;
  *                  1 = they run on a side stream of the plan, followed there

@@ -64,6 +64,15 @@ template <> struct SplitGeo32xK<726, 2> { using G = JGeo<726, 23, 256, 256, 4096
 template <int N> constexpr bool kSplit32 = (N == 351 || N == 726);
 template <int N> constexpr bool kSplit64 = (N == 176 || N == 363);
 
+// The CTA's next task: its first is its own number, the others come from the
+// counter (null where every task has a CTA), which starts at zero.
+__device__ __forceinline__ int nextTask(unsigned *counter, int ntasks, int *s_task) {
+    if (!counter) return ntasks;
+    if (threadIdx.x == 0) *s_task = (int)(gridDim.x + atomicAdd(counter, 1u));
+    __syncthreads();
+    return *s_task;
+}
+
 // Where an item's values go.  As an offset from `out` in either case, so that
 // the compiler still sees global memory (generic stores cost 10 %).
 __device__ __forceinline__ char *itemOut(const BatchItem &I, char *out) {
@@ -152,12 +161,7 @@ k_batch32(const DevParams32 *__restrict__ params, uint32_t *__restrict__ states,
     __shared__ __align__(16) uint32_t sbuf[MODE == -2 ? 4 : B];
     uint32_t *const buf = MODE == -2 ? g_mix32 : sbuf;
     __shared__ int s_task;
-    for (;;) {
-        if (threadIdx.x == 0) s_task = (int)atomicAdd(counter, 1u);
-        __syncthreads();
-        const int t = s_task;
-        __syncthreads();
-        if (t >= ntasks) break;
+    for (int t = blockIdx.x; t < ntasks; t = nextTask(counter, ntasks, &s_task)) {
         const BatchTask T = tasks[t];
         Lane32 L;
         L.load(params[T.pidx], threadIdx.x & 31);
@@ -224,12 +228,7 @@ k_batch32xk(const DevParams32 *__restrict__ params, uint32_t *__restrict__ state
     __shared__ int s_task;
     (void)polys;
     (void)nwords;
-    for (;;) {
-        if (threadIdx.x == 0) s_task = (int)atomicAdd(counter, 1u);
-        __syncthreads();
-        const int t = s_task;
-        __syncthreads();
-        if (t >= ntasks) break;
+    for (int t = blockIdx.x; t < ntasks; t = nextTask(counter, ntasks, &s_task)) {
         const BatchTask TK = tasks[t];
         Lane32 L;
         L.load(params[TK.pidx], threadIdx.x & 31);
@@ -303,12 +302,7 @@ k_batch64(const DevParams64 *__restrict__ params, uint64_t *__restrict__ states,
     __shared__ __align__(16) uint64_t sbuf[MODE == -2 ? 4 : B];
     uint64_t *const buf = MODE == -2 ? g_mix64 : sbuf;
     __shared__ int s_task;
-    for (;;) {
-        if (threadIdx.x == 0) s_task = (int)atomicAdd(counter, 1u);
-        __syncthreads();
-        const int t = s_task;
-        __syncthreads();
-        if (t >= ntasks) break;
+    for (int t = blockIdx.x; t < ntasks; t = nextTask(counter, ntasks, &s_task)) {
         const BatchTask T = tasks[t];
         Lane64 L;
         L.load(params[T.pidx], threadIdx.x & 31);
@@ -368,12 +362,7 @@ k_batch64x2(const DevParams64 *__restrict__ params, uint64_t *__restrict__ state
     __shared__ int s_task;
     (void)polys;
     (void)nwords;
-    for (;;) {
-        if (threadIdx.x == 0) s_task = (int)atomicAdd(counter, 1u);
-        __syncthreads();
-        const int t = s_task;
-        __syncthreads();
-        if (t >= ntasks) break;
+    for (int t = blockIdx.x; t < ntasks; t = nextTask(counter, ntasks, &s_task)) {
         const BatchTask TK = tasks[t];
         Lane64 L;
         L.load(params[TK.pidx], threadIdx.x & 31);
@@ -436,7 +425,7 @@ static cudaError_t resident(K kern, int tn, int *grid, size_t smem = 0) {
     return cudaSuccess;
 }
 
-// work counter reset -> persistent kernel
+// work counter reset (if tasks outnumber the CTAs) -> persistent kernel
 template <typename W, class K, class P>
 static cudaError_t go(K kern, int tn, const BatchLaunch &b, const P *params, W *states,
                       cudaStream_t s, size_t smem = 0) {
@@ -446,10 +435,13 @@ static cudaError_t go(K kern, int tn, const BatchLaunch &b, const P *params, W *
         if (e != cudaSuccess) return e;
     }
     if (grid > b.ntasks) grid = b.ntasks;
-    cudaError_t e = cudaMemsetAsync(b.counter, 0, sizeof(unsigned), s);
-    if (e != cudaSuccess) return e;
+    unsigned *counter = grid < b.ntasks ? b.counter : nullptr;
+    if (counter) {
+        cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned), s);
+        if (e != cudaSuccess) return e;
+    }
     kern<<<grid, tn, smem, s>>>(params, states, b.tasks, b.ntasks, b.items,
-                             static_cast<char *>(b.out), b.counter, static_cast<W *>(b.stage),
+                             static_cast<char *>(b.out), counter, static_cast<W *>(b.stage),
                              b.polys, b.nwords, static_cast<W *>(b.prewin));
     return cudaGetLastError();
 }

@@ -165,8 +165,9 @@ struct T32 {
                              W *dst, int stride, const JumpPart *d, int nd, cudaStream_t s) {
         return launchJumpParts32(mexp, p, st, polys, nw, dst, stride, d, nd, s);
     }
-    static cudaError_t windows(const W *gen, W *win, int n, int stride, int nwin, cudaStream_t s) {
-        return launchChunkWindows32(gen, win, n, stride, nwin, s);
+    static cudaError_t fan(int mexp, const DP *p, const W *st, const uint32_t *polys, int nw,
+                           W *dst, int stride, const JumpPart *d, int n, int cs, cudaStream_t s) {
+        return launchJumpFan32(mexp, p, st, polys, nw, dst, stride, d, n, cs, s);
     }
     static int resident(int mexp, bool split, int core) {
         return batchResident32(mexp, split, core);
@@ -218,8 +219,9 @@ struct T64 {
                              W *dst, int stride, const JumpPart *d, int nd, cudaStream_t s) {
         return launchJumpParts64(mexp, p, st, polys, nw, dst, stride, d, nd, s);
     }
-    static cudaError_t windows(const W *gen, W *win, int n, int stride, int nwin, cudaStream_t s) {
-        return launchChunkWindows64(gen, win, n, stride, nwin, s);
+    static cudaError_t fan(int mexp, const DP *p, const W *st, const uint32_t *polys, int nw,
+                           W *dst, int stride, const JumpPart *d, int n, int cs, cudaStream_t s) {
+        return launchJumpFan64(mexp, p, st, polys, nw, dst, stride, d, n, cs, s);
     }
     static int resident(int mexp, bool split, int core) {
         return batchResident64(mexp, split, core);
@@ -1136,12 +1138,11 @@ struct SingleFill {
         size_t cap_win = 0;
         unsigned char *h_desc = nullptr, *d_desc = nullptr;  // tasks | items | parts
         size_t cap_desc = 0;
-        unsigned *d_counter = nullptr;
+        unsigned *d_counter = nullptr;  // more chunks than CTAs
         // what the uploaded descriptors describe
         size_t n = 0;
-        int kind = -9, parts = 0;
+        int kind = -9;
         int64_t chunk = 0;
-        const void *win = nullptr, *polys = nullptr;
         mtgp_gpu_plan *plan = nullptr;  // jump_parts = -1: a split plan
     } slot[2];
     cudaEvent_t done[2] = {nullptr, nullptr};

@@ -228,12 +228,15 @@ cudaError_t launchJumpParts32(int mexp, const DevParams32 *params, const uint32_
 cudaError_t launchJumpParts64(int mexp, const DevParams64 *params, const uint64_t *states,
                               const uint32_t *polys, int nwords, uint64_t *dst, int stride,
                               const JumpPart *parts, int nparts, cudaStream_t s);
-// nwin windows of `stride` words at win: window 0 = gen[0..n), the others
-// zero (the destinations of jump parts).
-cudaError_t launchChunkWindows32(const uint32_t *gen, uint32_t *win, int n, int stride, int nwin,
-                                 cudaStream_t s);
-cudaError_t launchChunkWindows64(const uint64_t *gen, uint64_t *win, int n, int stride, int nwin,
-                                 cudaStream_t s);
+// A fan of n jumps, each by a team of cs CTAs (8, 4, 2 or 1): window dst[D.dst]
+// = the window at D.src jumped by polys[D.poly] (copied, poly < 0); u0 and u1
+// are not used.  MEXP 11213 and 23209.
+cudaError_t launchJumpFan32(int mexp, const DevParams32 *params, const uint32_t *states,
+                            const uint32_t *polys, int nwords, uint32_t *dst, int stride,
+                            const JumpPart *jumps, int n, int cs, cudaStream_t s);
+cudaError_t launchJumpFan64(int mexp, const DevParams64 *params, const uint64_t *states,
+                            const uint32_t *polys, int nwords, uint64_t *dst, int stride,
+                            const JumpPart *jumps, int n, int cs, cudaStream_t s);
 // descs null: a row of jumps by the same polynomials, described by `row` (a
 // kernel argument, no upload).
 cudaError_t launchJump32(int mexp, const DevParams32 *params, uint32_t *states,

@@ -40,6 +40,35 @@ k_jump(const typename G::Tr::P *__restrict__ params, typename G::W *__restrict__
         for (int k = threadIdx.x; k < G::N; k += G::NT) states[D.dst + at + k] = seq[k];
 }
 
+// A team of CS CTAs per jump of one window by polynomials of their own: window
+// dst[D.dst] of each, polynomial D.poly (-1: a copy).
+template <class G, int CS>
+__global__ void __launch_bounds__(G::NT, G::MINB)
+k_jump_fan(const typename G::Tr::P *__restrict__ params, const typename G::W *__restrict__ states,
+           const uint32_t *__restrict__ polys, int nwords, typename G::W *__restrict__ dst,
+           int stride, const JumpPart *__restrict__ parts) {
+    using W = typename G::W;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const Team<CS> team;
+    W *seq = reinterpret_cast<W *>(smem);
+    W *jout = reinterpret_cast<W *>(smem + G::off_jout);
+    const JumpPart &D = parts[blockIdx.x / CS];
+    W *to = dst + (size_t)D.dst * stride;
+    if (D.poly < 0) {  // the whole team
+        if (team.rank == 0)
+            for (int k = threadIdx.x; k < G::N; k += G::NT) to[k] = states[D.src + k];
+        return;
+    }
+    typename G::Tr::Lane L;
+    L.load(params[D.pidx], threadIdx.x & 31);
+    for (int k = threadIdx.x; k < G::N; k += G::NT) seq[k] = states[D.src + k];
+    jumpSorted<G>(smem, L, polys + (size_t)D.poly * nwords, nwords, kJumpUnits * team.rank / CS,
+                  kJumpUnits * (team.rank + 1) / CS);
+    if constexpr (CS > 1) team.sync();
+    for (int k = team.rank * G::NT + threadIdx.x; k < G::N; k += CS * G::NT) to[k] = team.sum(jout + k);
+    if constexpr (CS > 1) team.sync();  // before any CTA ends
+}
+
 // One CTA per (jump, share of its rows): XOR-ed into the zeroed destination
 // window.
 template <class G>
@@ -129,6 +158,36 @@ cudaError_t launch(Ring<Tr, Geo>, const typename Tr::P *params, typename Tr::W *
     if (ndesc <= 0) return cudaSuccess;
     k_jump_ring<Tr, Geo><<<ndesc, Geo::NT, smem, s>>>(params, states, descs, row, nwords);
     return cudaGetLastError();
+}
+
+template <class G, int CS>
+cudaError_t launchFanTeam(const typename G::Tr::P *params, const typename G::W *states,
+                          const uint32_t *polys, int nwords, typename G::W *dst, int stride,
+                          const JumpPart *jumps, int n, cudaStream_t s) {
+    static std::atomic<size_t> seen[16];
+    cudaError_t e = allowSmem(k_jump_fan<G, CS>, G::kBytes, seen);
+    if (e != cudaSuccess) return e;
+    return launchTeams(k_jump_fan<G, CS>, n, CS, G::NT, G::kBytes, s, params, states, polys,
+                       nwords, dst, stride, jumps);
+}
+
+template <class G>
+cudaError_t launchFan(G, const typename G::Tr::P *params, const typename G::W *states,
+                      const uint32_t *polys, int nwords, typename G::W *dst, int stride,
+                      const JumpPart *jumps, int n, int cs, cudaStream_t s) {
+    if (n <= 0) return cudaSuccess;
+    if (cs >= 8) return launchFanTeam<G, 8>(params, states, polys, nwords, dst, stride, jumps, n, s);
+    if (cs >= 4) return launchFanTeam<G, 4>(params, states, polys, nwords, dst, stride, jumps, n, s);
+    if (cs >= 2) return launchFanTeam<G, 2>(params, states, polys, nwords, dst, stride, jumps, n, s);
+    return launchFanTeam<G, 1>(params, states, polys, nwords, dst, stride, jumps, n, s);
+}
+
+// single fills are split only where the jump kernel sorts
+template <class Tr, class Geo>
+cudaError_t launchFan(Ring<Tr, Geo>, const typename Tr::P *, const typename Tr::W *,
+                      const uint32_t *, int, typename Tr::W *, int, const JumpPart *, int, int,
+                      cudaStream_t) {
+    return cudaErrorInvalidValue;
 }
 
 template <class G>
@@ -232,35 +291,26 @@ cudaError_t launchJumpParts64(int mexp, const DevParams64 *params, const uint64_
     return cudaErrorInvalidValue;
 }
 
-namespace {
-
-// Block c: win[c] = the generator's window for c = 0, zero otherwise (the
-// jump parts XOR into windows 1..).
-template <typename W>
-__global__ void __launch_bounds__(128)
-k_chunk_windows(const W *__restrict__ gen, W *__restrict__ win, int n, int stride) {
-    const size_t c = blockIdx.x;
-    W *dst = win + c * (size_t)stride;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) dst[k] = c ? W(0) : gen[k];
+cudaError_t launchJumpFan32(int mexp, const DevParams32 *params, const uint32_t *states,
+                            const uint32_t *polys, int nwords, uint32_t *dst, int stride,
+                            const JumpPart *jumps, int n, int cs, cudaStream_t s) {
+#define X(M, G)                                                                                 \
+    if (mexp == M)                                                                             \
+        return launchFan(UNWRAP(G)(), params, states, polys, nwords, dst, stride, jumps, n, cs, s);
+    MTGP_JGEO32(X)
+#undef X
+    return cudaErrorInvalidValue;
 }
 
-template <typename W>
-cudaError_t chunkWindows(const W *gen, W *win, int n, int stride, int nwin, cudaStream_t s) {
-    if (nwin <= 0 || n <= 0 || n > stride) return cudaErrorInvalidValue;
-    k_chunk_windows<W><<<nwin, 128, 0, s>>>(gen, win, n, stride);
-    return cudaGetLastError();
-}
-
-}  // namespace
-
-cudaError_t launchChunkWindows32(const uint32_t *gen, uint32_t *win, int n, int stride, int nwin,
-                                 cudaStream_t s) {
-    return chunkWindows(gen, win, n, stride, nwin, s);
-}
-
-cudaError_t launchChunkWindows64(const uint64_t *gen, uint64_t *win, int n, int stride, int nwin,
-                                 cudaStream_t s) {
-    return chunkWindows(gen, win, n, stride, nwin, s);
+cudaError_t launchJumpFan64(int mexp, const DevParams64 *params, const uint64_t *states,
+                            const uint32_t *polys, int nwords, uint64_t *dst, int stride,
+                            const JumpPart *jumps, int n, int cs, cudaStream_t s) {
+#define X(M, G)                                                                                 \
+    if (mexp == M)                                                                             \
+        return launchFan(UNWRAP(G)(), params, states, polys, nwords, dst, stride, jumps, n, cs, s);
+    MTGP_JGEO64(X)
+#undef X
+    return cudaErrorInvalidValue;
 }
 
 }  // namespace mtgp

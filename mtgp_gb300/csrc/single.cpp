@@ -8,11 +8,10 @@ namespace {
 // n successive values of one generator.  A fill of at least kSplitFillMin
 // values, on an exponent with GF(2) jumps, is cut into chunks: chunk c starts
 // from the generator's window jumped by X^(c * chunk) mod chi.  Those windows
-// are made first, every jump's correlation split over several CTAs
-// (k_jump_part, a range of the jump kernel's tap chunks each), from
-// polynomials kept on the device for the chunk length; then one batched
-// launch runs every chunk from its window on the two-word core, with no jump
-// inside it, and the window after the last chunk becomes the generator's.
+// are made first, every jump by a team of CTAs (k_jump_fan), from polynomials
+// kept on the device for the chunk length; then one batched launch runs every
+// chunk from its window on the two-word core, with no jump inside it, and the
+// last chunk leaves its final window in the generator: two launches in all.
 // A 2^20-value fill takes 0.035 ms this way (0.41 ms on one CTA), 2^25 values
 // 0.09 ms.  Smaller fills,
 // and fills issued while the stream is being captured, run on one CTA.  The
@@ -136,14 +135,14 @@ int fillSingle(Obj *h, int kind, void *out, size_t n, void *s) {
     }
     if (!L.d_counter) CK(devMalloc(&L.d_counter, sizeof(unsigned)), "devMalloc(counter)");
     W *win = static_cast<W *>(L.d_win);
-    const int parts = jumpParts(P.tune, nch - 1, sms);
-    const int nparts = (nch - 1) * parts;
+    // CTAs per chunk-start jump: a power of two
+    int team = kMaxJumpParts;
+    while (team > jumpParts(P.tune, nch - 1, sms - sms / 8)) team /= 2;
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
     const size_t off_items = al(sizeof(BatchTask) * (size_t)nch);
     const size_t off_parts = off_items + al(sizeof(BatchItem) * (size_t)nch);
-    const size_t bytes = off_parts + sizeof(JumpPart) * (size_t)nparts;
-    if (L.n != n || L.kind != kind || L.chunk != chunk || L.parts != parts || L.win != L.d_win ||
-        L.polys != F.d_polys) {
+    const size_t bytes = off_parts + sizeof(JumpPart) * (size_t)nch;
+    if (L.n != n || L.kind != kind || L.chunk != chunk) {
         L.n = 0;
         if (bytes > L.cap_desc) {
             cudaFreeHost(L.h_desc);
@@ -164,36 +163,27 @@ int fillSingle(Obj *h, int kind, void *out, size_t n, void *s) {
             t[c].nitems = 1;
             t[c].pidx = P.hpidx[0];
             t[c].j0 = t[c].j1 = -1;
-            t[c].wb = c == nch - 1 ? kWbStream : kWbNone;
+            t[c].wb = c == nch - 1 ? 0 : kWbNone;  // slot 0: the generator
             it[c] = BatchItem{};
             it[c].out_off = (uint64_t)c * (uint64_t)chunk * sizeof(W);
             it[c].count = c == nch - 1 ? n - (uint64_t)c * (uint64_t)chunk : (uint64_t)chunk;
             it[c].kind = kind;
         }
-        for (int c = 1; c < nch; c++)
-            for (int q = 0; q < parts; q++) {
-                JumpPart &d = jp[(size_t)(c - 1) * parts + q];
-                d = JumpPart{};
-                d.src = 0;
-                d.poly = c - 1;
-                d.dst = c;
-                d.pidx = P.hpidx[0];
-                d.u0 = (int16_t)partChunk(q, kJumpUnits, parts);
-                d.u1 = (int16_t)partChunk(q + 1, kJumpUnits, parts);
-            }
+        for (int c = 0; c < nch; c++) {
+            jp[c] = JumpPart{};
+            jp[c].poly = c - 1;  // -1: the generator's own window
+            jp[c].dst = c;
+            jp[c].pidx = P.hpidx[0];
+        }
         CK(cudaMemcpyAsync(L.d_desc, L.h_desc, bytes, cudaMemcpyHostToDevice, S(s)),
            "upload fill descriptors");
         L.n = n;
         L.kind = kind;
         L.chunk = chunk;
-        L.parts = parts;
-        L.win = L.d_win;
-        L.polys = F.d_polys;
     }
 
-    CK(T::windows(P.d_states, win, P.size, (int)stride, nch, S(s)), "chunk windows");
-    CK(T::parts(P.sh.mexp, P.d_params, win, F.d_polys, pw, win, (int)stride,
-                reinterpret_cast<const JumpPart *>(L.d_desc + off_parts), nparts, S(s)),
+    CK(T::fan(P.sh.mexp, P.d_params, P.d_states, F.d_polys, pw, win, (int)stride,
+              reinterpret_cast<const JumpPart *>(L.d_desc + off_parts), nch, team, S(s)),
        "chunk-start jumps");
     BatchLaunch b{};
     b.mexp = P.sh.mexp;
@@ -207,10 +197,8 @@ int fillSingle(Obj *h, int kind, void *out, size_t n, void *s) {
     b.items = reinterpret_cast<const BatchItem *>(L.d_desc + off_items);
     b.out = out;
     b.counter = L.d_counter;
+    b.stage = P.d_states;  // the last chunk's final window is the generator's
     CK(T::batch(b, P.d_params, win, S(s)), "chunks");
-    CK(cudaMemcpyAsync(P.d_states, win + (size_t)(nch - 1) * stride, sizeof(W) * (size_t)P.size,
-                       cudaMemcpyDeviceToDevice, S(s)),
-       "window after the last chunk");
     CK(cudaEventRecord(F.done[i], S(s)), "record fill");
     F.next ^= 1;
     return MTGP_OK;
