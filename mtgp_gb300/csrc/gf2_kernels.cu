@@ -295,8 +295,8 @@ cudaError_t launchGatherPow2(const uint32_t *blk, size_t tw, int W, int n, uint3
     return cudaGetLastError();
 }
 
-static cudaError_t powOps(const PowOp *ops, const FewOps &few, int n, const uint32_t *scratch,
-                          int W, cudaStream_t s, int window) {
+static cudaError_t powOps(const PowOp *ops, const FewOps &few, bool chains, int n,
+                          const uint32_t *scratch, int W, cudaStream_t s, int window) {
     if (n <= 0) return cudaSuccess;
     if (!powOpsFits(W)) return cudaErrorInvalidValue;
     const bool wide = window != 2 && powSmemWords<4>(W, 1) * 4 <= kPowSmemMax;
@@ -306,7 +306,7 @@ static cudaError_t powOps(const PowOp *ops, const FewOps &few, int n, const uint
     // few: a cluster each (one product 56 -> 31 us)
     const bool pairs = wide && n > sms && powSmemWords<4>(W, 3) * 4 <= kPowSmemPair;
     const int team = wide ? teamSize(n, sms) : 1;
-    const bool keep = pairs || (wide && powSmemWords<4>(W, 3) * 4 <= kPowSmemMax);
+    const bool keep = pairs || (wide && chains && powSmemWords<4>(W, 3) * 4 <= kPowSmemMax);
     const size_t smem = 4 * (wide ? powSmemWords<4>(W, keep ? 3 : 1) : powSmemWords<2>(W, 1));
     auto kern = pairs ? k_powops<4, 512, 1>
               : team == 8 ? k_powops<4, 1024, 8>
@@ -324,15 +324,19 @@ static cudaError_t powOps(const PowOp *ops, const FewOps &few, int n, const uint
 
 cudaError_t launchPowOps(const PowOp *ops, int n, const uint32_t *scratch, int W,
                          cudaStream_t s, int window) {
-    return powOps(ops, FewOps{}, n, scratch, W, s, window);
+    return powOps(ops, FewOps{}, false, n, scratch, W, s, window);
 }
 
 cudaError_t launchFewPowOps(const PowOp *host_ops, int n, const uint32_t *scratch, int W,
                             cudaStream_t s, int window) {
     if (n > kFewOps) return cudaErrorInvalidValue;
     FewOps few{};
-    for (int k = 0; k < n; k++) few.op[k] = host_ops[k];
-    return powOps(nullptr, few, n, scratch, W, s, window);
+    bool chains = false;
+    for (int k = 0; k < n; k++) {
+        few.op[k] = host_ops[k];
+        chains = chains || host_ops[k].nsrc > 2;
+    }
+    return powOps(nullptr, few, chains, n, scratch, W, s, window);
 }
 
 }  // namespace mtgp

@@ -908,6 +908,17 @@ struct Pool {
         if (rc) return rc;
         const int W = polyWords();
         PowSchedule sch;
+        if (n <= kFewOps) {
+            // a chain each, in one launch without upload or scratch: for one
+            // exponent the tree's allocation alone took longer than its four
+            // more products in turn
+            powSchedule(steps, n, 1, sch);
+            std::vector<PowOp> ops;
+            powOps(sch, [t](int) { return t; }, out, nullptr, chideg[k], ops);
+            CK(launchFewPowOps(ops.data(), n, nullptr, W, S(s), tune.poly_window),
+               "jump polynomials");
+            return MTGP_OK;
+        }
         powSchedule(steps, n, powWidth(), sch);
         unsigned char *d = nullptr;
         const size_t ops_bytes = (sizeof(PowOp) * (size_t)sch.steps() + 255) & ~size_t(255);
