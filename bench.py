@@ -49,10 +49,15 @@ L2_BYTES = 129 * 2 ** 20
 # of one launch each (dram__bytes_read.sum + dram__bytes_write.sum), keyed
 # by the captured plan's (core, split chunk, grid, windows jumped ahead)
 CAPTURED_TRAFFIC = {
-    (2, 393216, 760, 184): {
-        "bytes": 1677.8e6 + 6.85e6 + 0.52e6,
-        "source": "ncu capture of k_batch32xk<2> + k_jump_part5, one launch each, this plan "
-                  "(profiles/bench_default_plan_k_batch32xk2_k_jump_part5.md)"},
+    (2, 655360, 0, 53): {
+        "bytes": 1677.5e6 + 6.67e6 + 0.19e6,
+        "source": "ncu capture of k_batch32xk<2> + k_jump_part, one launch each, this plan "
+                  "(profiles/k_jump_and_k_batch32xk2_4096_substreams.md)"},
+    # the same tasks on 760 CTAs instead of 608: the same loads and stores
+    (2, 655360, 760, 53): {
+        "bytes": 1677.5e6 + 6.67e6 + 0.19e6,
+        "source": "ncu capture of k_batch32xk<2> + k_jump_part, one launch each, the same tasks on "
+                  "608 CTAs (profiles/k_jump_and_k_batch32xk2_4096_substreams.md)"},
 }
 METRIC = "batched MTGP32-11213 output GB/s"
 WORKLOAD = ("batched: mtgp32_params_fast_11213[0], seed 1234, 4096 substreams j*3^162 "
