@@ -127,6 +127,12 @@ constexpr int mixBlocks(int blocks, size_t smem) {
     return blocks < by_smem ? blocks : by_smem;
 }
 
+// Threads per SM that fix a one-word kernel's registers: 1280, 48 registers,
+// where that leaves five CTAs or more (plans take four; with 2048, 32 registers,
+// the tempering behind the recursion spilled: 4000 mixed requests 84 us, 80
+// with 1280), else 2048.
+constexpr int oneWordThreads(int tn, bool split) { return split || tn <= 256 ? 1280 : 2048; }
+
 template <int N, int TN, int B, int KIND>
 __device__ __noinline__ void mix32(Lane32 L, uint64_t n, char *o) {
     using OT = typename Out32<(KIND < 0 ? 0 : KIND)>::T;
@@ -151,8 +157,8 @@ __device__ __noinline__ void mix64(Lane64 L, uint64_t n, char *o) {
 // B words).  SPLIT: tasks may start with a jump.
 template <int N, int TN, int B, int MODE, bool SPLIT>
 __global__ void __launch_bounds__(TN, MODE == -2
-                                         ? mixBlocks((SPLIT ? 1280 : 2048) / TN, sizeof(uint32_t) * B)
-                                         : (SPLIT ? 1280 : 2048) / TN)
+                                         ? mixBlocks(oneWordThreads(TN, SPLIT) / TN, sizeof(uint32_t) * B)
+                                         : oneWordThreads(TN, SPLIT) / TN)
 k_batch32(const DevParams32 *__restrict__ params, uint32_t *__restrict__ states,
           const BatchTask *__restrict__ tasks, int ntasks,
           const BatchItem *__restrict__ items, char *__restrict__ out,
@@ -292,8 +298,8 @@ k_batch32xk(const DevParams32 *__restrict__ params, uint32_t *__restrict__ state
 
 template <int N, int TN, int B, int MODE, bool SPLIT>
 __global__ void __launch_bounds__(TN, MODE == -2
-                                         ? mixBlocks((SPLIT ? 1280 : 2048) / TN, sizeof(uint64_t) * B)
-                                         : (SPLIT ? 1280 : 2048) / TN)
+                                         ? mixBlocks(oneWordThreads(TN, SPLIT) / TN, sizeof(uint64_t) * B)
+                                         : oneWordThreads(TN, SPLIT) / TN)
 k_batch64(const DevParams64 *__restrict__ params, uint64_t *__restrict__ states,
           const BatchTask *__restrict__ tasks, int ntasks,
           const BatchItem *__restrict__ items, char *__restrict__ out,

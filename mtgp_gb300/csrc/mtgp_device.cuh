@@ -182,47 +182,41 @@ __device__ __forceinline__ void compact(W *buf, uint32_t src) {
     __syncthreads();
 }
 
-// One sub-step for 32-bit words.  px = buf + base + t, py = px + pos.
-template <int N, int TN, int KIND, bool GUARD>
-__device__ __forceinline__ void sub32(uint32_t *px, const Lane32 &L, uint32_t mul1,
-                                      uint32_t otab,
-                                      typename Out32<(KIND < 0 ? 0 : KIND)>::T *o,
-                                      bool live) {
+// One sub-step for 32-bit words, px = buf + base + t, py = px + pos: the word
+// made (r) and the one that tempers it (t).  `meanwhile`, the outputs of the
+// sub-step before, runs behind the shared store (CoreK::sub says why).
+template <int N, class F>
+__device__ __forceinline__ void sub32(uint32_t *px, const Lane32 &L, uint32_t mul1, uint32_t &r,
+                                      uint32_t &t, F meanwhile) {
     const uint32_t *py = px + L.pos;
-    uint32_t x1 = px[0], x2 = px[1], y = py[0];
-    uint32_t x = (x1 & L.mask) ^ x2;
-    uint32_t yy = x ^ (x * mul1) ^ (y >> L.sh2);
-    uint32_t r = yy ^ lut(L.tbl, yy);
-    px[N] = r;
-    if constexpr (KIND >= 0) {
-        uint32_t tt = py[-1];
-        uint32_t ov = lut(otab, fold(tt));
-        if (!GUARD || live) *o = Out32<KIND>::conv(r, ov);
-    }
+    const uint32_t x1 = px[0], x2 = px[1], y = py[0], tt = py[-1];
+    const uint32_t x = (x1 & L.mask) ^ x2;
+    const uint32_t yy = x ^ (x * mul1) ^ (y >> L.sh2);
+    const uint32_t v = yy ^ lut(L.tbl, yy);
+    px[N] = v;
+    meanwhile();
+    r = v;
+    t = tt;
     __syncthreads();
 }
 
-template <int N, int TN, int KIND, bool GUARD>
-__device__ __forceinline__ void sub64(uint64_t *px, const Lane64 &L, uint32_t mul1,
-                                      uint32_t olo, uint32_t ohi,
-                                      typename Out64<(KIND < 0 ? 0 : KIND)>::T *o,
-                                      bool live) {
+template <int N, class F>
+__device__ __forceinline__ void sub64(uint64_t *px, const Lane64 &L, uint32_t mul1, uint64_t &r,
+                                      uint32_t &t, F meanwhile) {
     const uint64_t *py = px + L.pos;
-    uint64_t x1 = px[0], x2 = px[1], y = py[0];
-    uint64_t x = (x1 & L.mask) ^ x2;
+    const uint64_t x1 = px[0], x2 = px[1], y = py[0], tt = py[-1];
+    const uint64_t x = (x1 & L.mask) ^ x2;
     uint32_t xh = (uint32_t)(x >> 32), xl = (uint32_t)x;
     uint32_t yh = (uint32_t)(y >> 32), yl = (uint32_t)y;
     xh ^= xh * mul1;
     xl ^= xl * mul1;
     yh = xl ^ (yh >> L.sh2);
     yl = xh ^ (yl >> L.sh2);
-    uint64_t r = (((uint64_t)yh << 32) | yl) ^ lut64(L.tbl_lo, L.tbl_hi, yl);
-    px[N] = r;
-    if constexpr (KIND >= 0) {
-        uint64_t tt = py[-1];
-        uint64_t ov = lut64(olo, ohi, fold((uint32_t)tt));
-        if (!GUARD || live) *o = Out64<KIND>::conv(r, ov);
-    }
+    const uint64_t v = (((uint64_t)yh << 32) | yl) ^ lut64(L.tbl_lo, L.tbl_hi, yl);
+    px[N] = v;
+    meanwhile();
+    r = v;
+    t = (uint32_t)tt;
     __syncthreads();
 }
 
@@ -237,10 +231,20 @@ __device__ __forceinline__ void run32(uint32_t *buf, const Lane32 &L, uint32_t o
     const uint32_t mul1 = 1u << L.sh1;
     uint32_t *px = buf + t;
     auto *o = out + t;
+    uint32_t pr, pt;  // of the sub-step not yet written out
+    auto emit = [&](auto *to, bool live) {
+        if constexpr (KIND >= 0) {
+            const uint32_t ov = lut(otab, fold(pt));
+            if (live) *to = Out32<KIND>::conv(pr, ov);
+        }
+    };
     while (n >= (uint64_t)S * TN) {
 #pragma unroll
         for (int k = 0; k < S; k++)
-            sub32<N, TN, KIND, false>(px + k * TN, L, mul1, otab, o + k * TN, true);
+            sub32<N>(px + k * TN, L, mul1, pr, pt, [&] {
+                if (k > 0) emit(o + (k - 1) * TN, true);
+            });
+        emit(o + (S - 1) * TN, true);
         compact<uint32_t, N, TN>(buf, S * TN);
         n -= (uint64_t)S * TN;
         if constexpr (KIND >= 0) o += S * TN;
@@ -249,7 +253,10 @@ __device__ __forceinline__ void run32(uint32_t *buf, const Lane32 &L, uint32_t o
     if (rem == 0) return;
     const int subs = (rem + TN - 1) / TN;
     for (int k = 0; k < subs; k++)
-        sub32<N, TN, KIND, true>(px + k * TN, L, mul1, otab, o + k * TN, k * TN + t < rem);
+        sub32<N>(px + k * TN, L, mul1, pr, pt, [&] {
+            if (k > 0) emit(o + (k - 1) * TN, true);
+        });
+    emit(o + (subs - 1) * TN, (subs - 1) * TN + t < rem);
     compact<uint32_t, N, TN>(buf, (uint32_t)rem);
 }
 
@@ -262,10 +269,21 @@ __device__ __forceinline__ void run64(uint64_t *buf, const Lane64 &L, uint32_t o
     const uint32_t mul1 = 1u << L.sh1;
     uint64_t *px = buf + t;
     auto *o = out + t;
+    uint64_t pr;  // of the sub-step not yet written out
+    uint32_t pt;
+    auto emit = [&](auto *to, bool live) {
+        if constexpr (KIND >= 0) {
+            const uint64_t ov = lut64(olo, ohi, fold(pt));
+            if (live) *to = Out64<KIND>::conv(pr, ov);
+        }
+    };
     while (n >= (uint64_t)S * TN) {
 #pragma unroll
         for (int k = 0; k < S; k++)
-            sub64<N, TN, KIND, false>(px + k * TN, L, mul1, olo, ohi, o + k * TN, true);
+            sub64<N>(px + k * TN, L, mul1, pr, pt, [&] {
+                if (k > 0) emit(o + (k - 1) * TN, true);
+            });
+        emit(o + (S - 1) * TN, true);
         compact<uint64_t, N, TN>(buf, S * TN);
         n -= (uint64_t)S * TN;
         if constexpr (KIND >= 0) o += S * TN;
@@ -274,7 +292,10 @@ __device__ __forceinline__ void run64(uint64_t *buf, const Lane64 &L, uint32_t o
     if (rem == 0) return;
     const int subs = (rem + TN - 1) / TN;
     for (int k = 0; k < subs; k++)
-        sub64<N, TN, KIND, true>(px + k * TN, L, mul1, olo, ohi, o + k * TN, k * TN + t < rem);
+        sub64<N>(px + k * TN, L, mul1, pr, pt, [&] {
+            if (k > 0) emit(o + (k - 1) * TN, true);
+        });
+    emit(o + (subs - 1) * TN, (subs - 1) * TN + t < rem);
     compact<uint64_t, N, TN>(buf, (uint32_t)rem);
 }
 
