@@ -500,9 +500,11 @@ int mtgp32_gpu_batch_noalloc(const mtgp32_params_fast_t *params, int nparams,
  * pending requests first-come-first-served into batches of at most
  * `max_batch` requests (and an eighth of the budget, up to half under a
  * backlog), keeps up to `slots` (at most
- * 256) batches in flight on their own CUDA streams, and copies each result
- * to its destination when the batch completes.  A batch's outputs take one
- * block of the arena, placed in admission order; results kept in the arena
+ * 256) batches in flight on their own CUDA streams.  A result's destination
+ * in this device's memory (aligned to the value, within one allocation, apart
+ * from the batch's other destinations) is written while the batch runs, any
+ * other by a copy when it completes; leave it alone until the request is done.
+ * A batch's outputs take one block of the arena, placed in admission order; results kept in the arena
  * (mtgp_server_submit without destination) hold their part of a block until
  * released, so long-kept results fragment the arena.  Requests of one
  * stream run in submission order (a batch that holds a stream runs on the

@@ -3,18 +3,16 @@
 //
 // A batch is a list of tasks; a task is one stream and a chain of work items
 // (count, output kind, output byte offset) that continue that stream in
-// order.  The grid is sized to the number of CTAs the GPU keeps resident;
-// each CTA takes the next task from a device counter (tasks are sorted
-// longest-first on the host, so the long ones start first), loads the
-// stream's window into shared memory, runs the items with a generation core,
-// and writes the advanced window back.
+// order.  The grid is a few CTAs per SM (planCtas), or what the caller asks
+// for; a CTA's first task is its own number and it takes the next ones from a
+// device counter (tasks are sorted longest-first on the host, so the long ones
+// start first), loads the stream's window into shared memory, runs the items
+// with a generation core, and writes the advanced window back.
 //
 // Long requests are split into chunks that run on different CTAs: chunk c
-// starts from the stream's window jumped ahead by its offset (X^off mod chi,
-// applied inside the chunk's CTA with jump_device.cuh).  The jump is
-// ALU-bound while generation is bound by the shared-memory data pipe, so the
-// jumps of some CTAs overlap the generation of the others.  Only the last
-// chunk keeps its final window, in a staging slot that k_unstage copies back
+// starts from the stream's window jumped ahead by its offset (X^off mod chi),
+// made before the launch by jump_kernels.cu, or inside the chunk's CTA with
+// jump_device.cuh (jump_parts = -1).  Only the last chunk keeps its final window, in a staging slot that k_unstage copies back
 // after the launch, so no chunk can read a window that another chunk has
 // already advanced.
 //
