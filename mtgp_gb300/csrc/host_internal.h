@@ -187,6 +187,9 @@ struct T32 {
     // a string byte as the reference adds it to the state: a signed char
     // (its behaviour on x86-64), whatever the host's char signedness
     static W strKey(char c) { return (W)(int)(signed char)c; }
+    // all float table entries in [1, 2): what the 64-bit two-word core needs
+    // for the kinds that subtract; the 32-bit cores take any table
+    static bool unitTables(const HP &) { return true; }
 };
 
 struct T64 {
@@ -239,6 +242,11 @@ struct T64 {
         return launchKeyed64(p, pi, keys, koff, st, n, size, stride, nullptr);
     }
     static W strKey(char c) { return (W)(int64_t)(int)(signed char)c; }
+    static bool unitTables(const HP &p) {
+        for (uint64_t e : p.dbl_tmp_tbl)
+            if (e >> 52 != 0x3ff) return false;
+        return true;
+    }
 };
 
 template <class T>
@@ -286,6 +294,9 @@ struct Pool {
     // plan needs is the plan's own or thread-local.
     std::recursive_mutex cache_mu;
     Tuning tune = tuningDefaults();  // this pool's tuning knobs
+    bool unit = true;                // T::unitTables of every parameter set
+    // The generation core for an output kind.
+    int coreFor(int kind) const { return !unit && kind >= 2 ? 1 : tune.core; }
 
     ~Pool() {
         if (cache_stream) cudaStreamSynchronize(cache_stream);
@@ -329,7 +340,10 @@ struct Pool {
             hpidx[i] = k;
         }
         std::vector<typename T::DP> dp(np);
-        for (int k = 0; k < np; k++) toDev(params[k], &dp[k]);
+        for (int k = 0; k < np; k++) {
+            toDev(params[k], &dp[k]);
+            unit = unit && T::unitTables(params[k]);
+        }
         CK(devMalloc(&d_params, sizeof(typename T::DP) * np), "devMalloc(params)");
         CK(devMalloc(&d_pidx, sizeof(int) * n), "devMalloc(pidx)");
         CK(devMalloc(&d_states, sizeof(W) * (size_t)stride * n), "devMalloc(states)");
@@ -418,7 +432,7 @@ struct Pool {
         int rc = checkKind(kind);
         if (!rc) rc = checkOut(out, n);
         if (rc) return rc;
-        CK(T::gen(sh.mexp, kind, d_params, d_pidx, d_states, count, out, n, n, S(s), tune.core),
+        CK(T::gen(sh.mexp, kind, d_params, d_pidx, d_states, count, out, n, n, S(s), coreFor(kind)),
            "generate");
         return MTGP_OK;
     }
@@ -429,7 +443,7 @@ struct Pool {
         if (!rc && kind >= 0) rc = checkOut(out, n);
         if (rc) return rc;
         CK(T::gen(sh.mexp, kind, d_params, d_pidx + i, d_states + (size_t)i * stride, 1, out, n, n,
-                  S(s), tune.core),
+                  S(s), coreFor(kind)),
            "generate");
         return MTGP_OK;
     }

@@ -89,6 +89,37 @@ struct Out64 {
     }
 };
 
+// Out64 for parameter sets whose double table entries are all in [1, 2): the
+// subtraction of the last three kinds in integers.  x - 1.0 (or 2.0 - x, FLIP)
+// of x = 1 + m 2^-52 is q 2^-52, q = m or 2^52 - m, exactly: its leading one
+// goes to bit 52 and the exponent follows.  A double subtraction takes an SM 16
+// cycles a warp here (100 x 200000 values by a plan: 175 us with it, 112 so).
+// The two-word core; other sets take the one-word core for these kinds
+// (Pool::coreFor).
+template <bool FLIP>
+__device__ __forceinline__ double unitDiff(uint64_t v) {
+    const uint64_t m = v & 0xfffffffffffffULL;
+    const uint64_t q = FLIP ? (uint64_t(1) << 52) - m : m;
+    const int s = __clzll((long long)q) - 11;
+    const uint64_t r = (q << s) + ((uint64_t)(uint32_t)(1022 - s) << 52);
+    return __longlong_as_double(q ? (long long)r : 0LL);
+}
+
+template <int KIND>
+struct OutUnit64 : Out64<KIND> {
+    __device__ __forceinline__ static typename Out64<KIND>::T conv(uint64_t r, uint64_t o) {
+        if constexpr (KIND == MTGP_KIND_CLOSE_OPEN) {
+            return unitDiff<false>((r >> 12) ^ o);
+        } else if constexpr (KIND == MTGP_KIND_OPEN_CLOSE) {
+            return unitDiff<true>((r >> 12) ^ o);
+        } else if constexpr (KIND == MTGP_KIND_OPEN_OPEN) {
+            return unitDiff<false>(((r >> 12) | 1u) ^ o);
+        } else {
+            return Out64<KIND>::conv(r, o);
+        }
+    }
+};
+
 // Per-lane copies of a generator's constants: lane l holds entry l & 15 of
 // the recursion table, the tempering table and the float tempering table.
 struct Lane32 {

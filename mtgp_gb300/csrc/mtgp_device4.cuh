@@ -48,10 +48,11 @@ using Geo4 = GeoK<N, W, B, 4>;
 
 // The shared buffer (words) of a kernel that runs few CTAs per SM: 45 KB, 42
 // sub-steps before the window moves instead of 14 (the 128 generators: 521 ->
-// 490 us).  The batched kernels keep the short one (412 to 417 us against
+// 490 us); for 64-bit words 21, whose code is longer (200003 doubles in [0, 1)
+// of one generator: 220 us with 42, 134 with 21).  The batched kernels keep the short one (412 to 417 us against
 // 416 on 4096 lognormal streams, 449 against 419 on 64-bit words).
 template <int N, int B>
-constexpr int kLongBuf = N == 351 ? 11264 : N == 176 ? 5632 : B;
+constexpr int kLongBuf = N == 351 ? 11264 : N == 176 ? 2944 : B;
 
 // Index of sequence position j in the K-plane buffer.
 template <int PW, int K = 4>

@@ -118,7 +118,7 @@ struct Core64x2 {
         if constexpr (KIND >= 0) {
             OT v[K];
 #pragma unroll
-            for (int c = 0; c < K; c++) v[c] = Out64<KIND>::conv(P.r[c], lut64(olo, ohi, fold(P.t[c])));
+            for (int c = 0; c < K; c++) v[c] = OutUnit64<KIND>::conv(P.r[c], lut64(olo, ohi, fold(P.t[c])));
             if (!GUARD || valid >= K) {
                 *reinterpret_cast<typename VO::V *>(o) = VO::make(v);
             } else {
@@ -177,7 +177,7 @@ struct Core64x2 {
                 if constexpr (KIND >= 0) ov = lut64(olo, ohi, fold((uint32_t)tt));
                 if (t == 0) {
                     buf[at(N)] = r;
-                    if constexpr (KIND >= 0) out[0] = Out64<(KIND < 0 ? 0 : KIND)>::conv(r, ov);
+                    if constexpr (KIND >= 0) out[0] = OutUnit64<(KIND < 0 ? 0 : KIND)>::conv(r, ov);
                 }
             }
             __syncthreads();

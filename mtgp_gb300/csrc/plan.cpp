@@ -50,7 +50,7 @@ int makePlan(Pool<T> &P, const mtgp_work_item_t *items, int nitems, mtgp_gpu_pla
             if (it.count) addKind(it.kind);
         }
     }
-    int core = force_core ? force_core : kinds == -2 ? 1 : P.tune.core;
+    int core = force_core ? force_core : kinds == -2 ? 1 : P.coreFor(kinds);
     // 64-bit cores: two words per thread (knob 2 or 4) or one; the two-word
     // kernel has no jump code, so plans with in-kernel jumps (jump_parts =
     // -1) take the one-word core

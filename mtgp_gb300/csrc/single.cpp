@@ -188,8 +188,8 @@ int fillSingle(Obj *h, int kind, void *out, size_t n, void *s) {
     BatchLaunch b{};
     b.mexp = P.sh.mexp;
     b.mode = kind;
-    b.grid = std::min(nch, T::resident(P.sh.mexp, false, 2));
-    b.core = 2;
+    b.core = P.unit || kind < 2 ? 2 : 1;
+    b.grid = std::min(nch, T::resident(P.sh.mexp, false, b.core));
     b.split = false;
     b.nwords = pw;
     b.tasks = reinterpret_cast<const BatchTask *>(L.d_desc);
@@ -291,6 +291,7 @@ int importSingle(Obj *h, const typename T::Fast *src) {
     CK(cudaDeviceSynchronize(), "synchronize");
     CK(cudaMemcpy(h->pool.d_params, &dp, sizeof dp, cudaMemcpyHostToDevice), "upload params");
     h->pool.hparams[0] = src->params;
+    h->pool.unit = T::unitTables(src->params);
     h->pool.chideg[0] = -1;
     return h->pool.setWindows(win.data(), win.size());
 }
