@@ -130,27 +130,29 @@ struct Core64x2 {
     }
 
     // Sub-step k of a segment: two words per thread.  `meanwhile`, the tempering
-    // of the sub-step before, runs between its loads and their use: off the
-    // chain load - recursion - store - barrier that one generator's speed
-    // hangs on (2^25 values of one generator in 256 chunks: 151 -> 128 us; 144
-    // with the tempering after the stores, as the 32-bit core has it).
+    // of the sub-step before, is off the chain load - recursion - store -
+    // barrier that one generator's speed hangs on: at MEXP 11213, two warps, it
+    // runs between the loads and their use (2^25 values of one generator in 256
+    // chunks: 151 -> 128 us, 144 behind the stores), at the longer exponents
+    // behind the stores (200003 values at MEXP 44497: 60.4 us, 66.6 behind the
+    // loads, 64.7 where the words are made).
     template <class F>
     __device__ static __forceinline__ void sub(uint64_t *buf, const Idx &I, int k, const Lane64 &L,
                                                uint32_t mul1, Pend &P, F meanwhile) {
         const int d = k * G::STEP;
-        uint64_t xs[K + 1], ys[K + 1];
+        uint64_t xs[K + 1], ys[K + 1], r[K];
 #pragma unroll
         for (int c = 0; c <= K; c++) ys[c] = buf[I.y[c] + d];
 #pragma unroll
         for (int c = 0; c <= K; c++) xs[c] = buf[I.x[c] + d];
-        meanwhile();
+        if constexpr (N == 176) meanwhile();
 #pragma unroll
-        for (int c = 0; c < K; c++) {
-            P.r[c] = rec64(xs[c], xs[c + 1], ys[c + 1], L, mul1);
-            P.t[c] = (uint32_t)ys[c];
-        }
+        for (int c = 0; c < K; c++) r[c] = rec64(xs[c], xs[c + 1], ys[c + 1], L, mul1);
 #pragma unroll
-        for (int c = 0; c < K; c++) buf[I.w[c] + d] = P.r[c];
+        for (int c = 0; c < K; c++) buf[I.w[c] + d] = r[c];
+        if constexpr (N != 176) meanwhile();
+#pragma unroll
+        for (int c = 0; c < K; c++) P.r[c] = r[c], P.t[c] = (uint32_t)ys[c];
         __syncthreads();
     }
 
