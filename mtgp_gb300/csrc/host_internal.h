@@ -46,6 +46,15 @@ inline int cudaErr(cudaError_t e, const char *what) {
 
 inline cudaStream_t S(void *s) { return static_cast<cudaStream_t>(s); }
 
+// A call that cannot be part of a graph refuses a stream being captured before
+// it queues anything there: what is captured has not run when it returns.
+inline int notCapturing(void *s, const char *what) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(S(s), &cs), "capture status");
+    return cs == cudaStreamCaptureStatusNone ? MTGP_OK
+                                             : cudaErr(cudaErrorStreamCaptureUnsupported, what);
+}
+
 // Tuning knobs (mtgp_gpu_set_tuning).  split_chunk: 0 = automatic, < 0 =
 // never split long requests, > 0 = split into chunks of this many values.
 // batch_grid: 0 = automatic (planCtas() CTAs per SM, or every resident slot
@@ -963,14 +972,12 @@ struct Pool {
     // turn.  Not for a stream being captured.
     int jumpGpu(int i, uint64_t steps, void *s) {
         if (i < 0 || i >= count) return setErr(MTGP_ERR_INVALID, "stream %d out of range", i);
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        CK(cudaStreamIsCapturing(S(s), &cs), "capture status");
-        if (cs != cudaStreamCaptureStatusNone)
-            return cudaErr(cudaErrorStreamCaptureUnsupported, "jump");
+        int rc = notCapturing(s, "jump");
+        if (rc) return rc;
         const int W = polyWords();
         const int k = hpidx[i];
         const uint32_t *t = nullptr;
-        int rc = gpuPowTables(k, &t);
+        rc = gpuPowTables(k, &t);
         if (!rc) rc = ensureScratch((size_t)(1 + kPowMaxSrc) * W, 1);
         if (rc) return rc;
         PowSchedule sch;
@@ -1229,7 +1236,9 @@ struct mtgp_gpu_plan {
     const JumpPart *d_parts = nullptr;
     void *d_prewin = nullptr;
     size_t cap_prewin = 0;
-    bool prewin_fresh = false;  // allocated, not yet zeroed
+    // the slots may hold something else than zeros: newly allocated, or left
+    // by a launch that failed
+    bool prewin_fresh = false;
     // jump_overlap: tasks [nmain, ntasks) start from pre-jumped windows and
     // run in a second persistent launch on `side`, after the jump parts
     // there, beside the launch of tasks [0, nmain) on the caller's stream
@@ -1273,7 +1282,7 @@ class SparePlan {
         plan_ = nullptr;
         return p;
     }
-    // p is idle on the GPU
+    // p is idle on the GPU, and its last launch, if any, was whole
     void give(mtgp_gpu_plan *p) {
         if (!p) return;
         for (void *b : p->retired_dev) cudaFree(b);

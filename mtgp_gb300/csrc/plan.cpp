@@ -436,6 +436,9 @@ int launchPlan(mtgp_gpu_plan *pl, void *out, void *s) {
         CK(cudaEventRecord(pl->fork, S(s)), "fork");
         CK(cudaStreamWaitEvent(pl->side, pl->fork, 0), "fork");
     }
+    // from the first parts on until the batched kernel, which zeroes the slots
+    // again, is queued: an error in between leaves them to be zeroed anew
+    pl->prewin_fresh = pl->npre > 0;
     if (pl->nparts) {  // the start windows jumped ahead of the launch, into zeroed slots
         using W = typename T::W;
         W *pre = static_cast<W *>(pl->d_prewin);
@@ -488,10 +491,8 @@ int launchPlan(mtgp_gpu_plan *pl, void *out, void *s) {
     } else {
         e = T::batch(b, P.d_params, P.d_states, S(s));
     }
-    if (e != cudaSuccess) {
-        pl->prewin_fresh = pl->npre > 0;  // the slots may hold jump parts: zero them again
-        return cudaErr(e, "batched launch");
-    }
+    if (e != cudaSuccess) return cudaErr(e, "batched launch");
+    pl->prewin_fresh = false;
     return MTGP_OK;
 }
 

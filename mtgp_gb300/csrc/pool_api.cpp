@@ -250,12 +250,18 @@ extern "C" {
     int mtgp##B##_gpu_pool_submit(mtgp##B##_gpu_pool_t *p, const mtgp_work_item_t *items,        \
                                   int nitems, void *out, void *s) {                              \
         if (!p) return setErr(MTGP_ERR_INVALID, "null pool");                                    \
+        int rc = notCapturing(s, "submit");                                                      \
+        if (rc) return rc;                                                                       \
         mtgp_gpu_plan_t *pl = p->spare.take();                                                   \
-        int rc = makePlan(p->pool, items, nitems, &pl);                                          \
+        rc = makePlan(p->pool, items, nitems, &pl);                                              \
         if (!rc) {                                                                               \
             rc = planLaunch(pl, out, s);                                                         \
             const cudaError_t e = cudaStreamSynchronize(S(s));                                   \
             if (!rc && e != cudaSuccess) rc = cudaErr(e, "batched launch");                      \
+            if (rc) { /* what was queued of it, on either stream, ends first */                  \
+                mtgp_gpu_plan_free(pl);                                                          \
+                return rc;                                                                       \
+            }                                                                                    \
         }                                                                                        \
         p->spare.give(pl);                                                                       \
         return rc;                                                                               \
