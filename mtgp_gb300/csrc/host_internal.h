@@ -726,6 +726,20 @@ struct Pool {
         }
         return MTGP_OK;
     }
+    // Drop every polynomial and table of the parameter sets (new ones follow).
+    // The device is idle.
+    void forgetPolys() {
+        chi.assign(hparams.size(), gf2::Poly());
+        chideg.assign(hparams.size(), -1);
+        mod.clear();
+        pow2.clear();
+        jcache.clear();
+        afill.keys.clear();  // a fill that nobody has taken yet
+        afill.busy = afill.submitted = false;
+        gpow.clear();
+        for (uint32_t *b : gpow_blocks) cudaFree(b);
+        gpow_blocks.clear();
+    }
     int gpuPowTables(int k, const uint32_t **out) {
         int rc = prepare({k});
         if (rc) return rc;
@@ -937,7 +951,7 @@ struct Pool {
             // more products in turn
             powSchedule(steps, n, 1, sch);
             std::vector<PowOp> ops;
-            powOps(sch, [t](int) { return t; }, out, nullptr, chideg[k], ops);
+            powOps(sch, [t](int) { return t; }, out, nullptr, sh.mexp, ops);
             CK(launchFewPowOps(ops.data(), n, nullptr, W, S(s), tune.poly_window),
                "jump polynomials");
             return MTGP_OK;
@@ -949,7 +963,7 @@ struct Pool {
         CK(devMallocAsync(reinterpret_cast<void **>(&d), bytes, S(s)), "devMallocAsync(products)");
         uint32_t *scratch = reinterpret_cast<uint32_t *>(d + ops_bytes);
         std::vector<PowOp> ops;
-        powOps(sch, [t](int) { return t; }, out, scratch, chideg[k], ops);
+        powOps(sch, [t](int) { return t; }, out, scratch, sh.mexp, ops);
         cudaError_t e = cudaMemcpyAsync(d, ops.data(), sizeof(PowOp) * ops.size(),
                                         cudaMemcpyHostToDevice, S(s));
         size_t first = 0;
@@ -984,7 +998,7 @@ struct Pool {
         powSchedule(&steps, 1, powWidth(), sch);
         std::vector<PowOp> ops;
         uint32_t *scratch = d_poly + W;  // a tree of eight factors has six inner products
-        powOps(sch, [t](int) { return t; }, d_poly, scratch, chideg[k], ops);
+        powOps(sch, [t](int) { return t; }, d_poly, scratch, sh.mexp, ops);
         size_t first = 0;
         for (const auto &lev : sch.levels) {
             CK(launchFewPowOps(ops.data() + first, (int)lev.size(), scratch, W, S(s),

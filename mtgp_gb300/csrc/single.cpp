@@ -290,9 +290,16 @@ int importSingle(Obj *h, const typename T::Fast *src) {
     toDev(src->params, &dp);
     CK(cudaDeviceSynchronize(), "synchronize");
     CK(cudaMemcpy(h->pool.d_params, &dp, sizeof dp, cudaMemcpyHostToDevice), "upload params");
+    // the jump polynomials depend on what the recursion reads of a set
+    const typename T::HP &was = h->pool.hparams[0], &now = src->params;
+    if (was.pos != now.pos || was.sh1 != now.sh1 || was.sh2 != now.sh2 || was.mask != now.mask ||
+        std::memcmp(was.tbl, now.tbl, sizeof now.tbl)) {
+        h->pool.forgetPolys();
+        h->fill.poly_chunk = 0;
+        h->fill.npolys = 0;
+    }
     h->pool.hparams[0] = src->params;
     h->pool.unit = T::unitTables(src->params);
-    h->pool.chideg[0] = -1;
     return h->pool.setWindows(win.data(), win.size());
 }
 

@@ -2,8 +2,8 @@
 // and with a log of what was queued, so that its error paths (a launch that
 // fails, a stream being captured) can be tested without a GPU.  Kernels do
 // nothing but what a test looks at: generation writes the parameter set's
-// `pos`, Berlekamp-Massey takes its polynomial from that, a product passes
-// its chi on.  Built by fake_gpu.py with the library's own .cpp files.
+// `pos`, Berlekamp-Massey takes its polynomial's last word from that, a product
+// passes the first word of its chi on.  Built by fake_gpu.py with the library's own .cpp files.
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -228,7 +228,7 @@ int batchResident64(int, bool, int) { return 1520; }
         for (int j = 0; j < nseq; j++) {                                                         \
             L[j] = n2 / 2;                                                                       \
             C[(size_t)j * nw] = 1;                                                               \
-            C[(size_t)j * nw + (n2 / 2 - 31) / 32] = (uint32_t)seqs[(size_t)j * n2];             \
+            C[(size_t)j * nw + n2 / 64] = (uint32_t)seqs[(size_t)j * n2];                        \
         }                                                                                        \
         return queued("launchBM" #B, s);                                                         \
     }                                                                                            \
@@ -271,7 +271,6 @@ cudaError_t launchMonomials(uint32_t *, size_t, int, int, int, cudaStream_t s) {
 cudaError_t launchGatherPow2(const uint32_t *, size_t, int, int, uint32_t *, cudaStream_t s) {
     return queued("launchGatherPow2", s);
 }
-// A product is its chi's first word.
 static cudaError_t pow(const PowOp *ops, int n, cudaStream_t s) {
     for (int k = 0; k < n; k++) {
         ops[k].dst[0] = ops[k].tab[0];
