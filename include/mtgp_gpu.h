@@ -503,7 +503,9 @@ int mtgp32_gpu_batch_noalloc(const mtgp32_params_fast_t *params, int nparams,
  * 256) batches in flight on their own CUDA streams.  A result's destination
  * in this device's memory (aligned to the value, within one allocation, apart
  * from the batch's other destinations) is written while the batch runs, any
- * other by a copy when it completes; leave it alone until the request is done.
+ * other by a copy when it completes.  No stream of the caller's is waited for:
+ * earlier work on a destination has to be done when its request is submitted,
+ * and the destination is left alone until the request is done.
  * A batch's outputs take one block of the arena, placed in admission order; results kept in the arena
  * (mtgp_server_submit without destination) hold their part of a block until
  * released, so long-kept results fragment the arena.  Requests of one
@@ -526,7 +528,8 @@ typedef struct mtgp_request {
 /* (In a replayed trace a request without destination is discarded when it
  * completes; mtgp_server_submit keeps such results instead.) */
 
-/* Either pool may be NULL (not both).  The pools must outlive the server. */
+/* Either pool may be NULL (not both).  The pools must outlive the server.
+ * Waits for the device, whose queued work may still make the pools' windows. */
 int mtgp_server_create(mtgp_server_t **out, mtgp32_gpu_pool_t *p32,
                        mtgp64_gpu_pool_t *p64, uint64_t budget_bytes,
                        int slots, int max_batch);

@@ -385,7 +385,8 @@ class Server:
 
     `submit` queues a request and returns its ticket; the values land in
     `dst` (a CUDA or CPU tensor of the pool's word size) once `wait(ticket)`
-    returns.  Without `dst` the result stays in the server's device arena:
+    returns (earlier work on `dst`, on any stream, has to be done before the
+    submit).  Without `dst` the result stays in the server's device arena:
     `result(ticket)` is a zero-copy view of it until `release(ticket)`."""
 
     def __init__(self, pool32=None, pool64=None, budget_bytes=1 << 30, slots=4, max_batch=4096):
@@ -466,10 +467,12 @@ class Server:
     def replay(self, requests, arrivals):
         """Submit `requests` (a REQUEST_DTYPE array) at `arrivals` (seconds
         from now) and drain; returns the wall time in seconds.  Results of
-        requests without destination are discarded at completion."""
+        requests without destination are discarded at completion.  Work queued
+        on the current stream (on the destinations) is waited for first."""
         req = np.ascontiguousarray(requests, dtype=REQUEST_DTYPE)
         arr = np.ascontiguousarray(arrivals, dtype=np.float64)
         assert len(req) == len(arr)
+        torch.cuda.current_stream().synchronize()
         wall = ctypes.c_double()
         check(lib().mtgp_server_replay(self.h, req.ctypes.data_as(ctypes.c_void_p),
                                        arr.ctypes.data_as(ctypes.c_void_p), len(arr),

@@ -534,6 +534,9 @@ int mtgp_server_create(mtgp_server_t **out, mtgp32_gpu_pool_t *p32, mtgp64_gpu_p
             e = cudaEventCreateWithFlags(&sl->ev, cudaEventDisableTiming | cudaEventBlockingSync);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sl->join, cudaEventDisableTiming);
     }
+    // the pools' windows may still be on their way on the streams that made
+    // them, for which the slots' own streams do not wait
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {
         mtgp_server_destroy(s);
         return mtgp::recordError(MTGP_ERR_CUDA, cudaGetErrorString(e));
