@@ -290,7 +290,9 @@ int mtgp32_gpu_pool_create_by_str(mtgp32_gpu_pool_t **out,
  * count <= 4^rows.  The jumps run on the GPU: the same rows in the same
  * order as the reference's table walk (cuda-sample/mtgp32-jump-kernel.cuh:
  * 383-423), so the windows are identical to it, but made by doubling (level
- * k jumps windows [0, 2^k) into [2^k, 2^(k+1))), one jump per substream. */
+ * k jumps windows [0, 2^k) into [2^k, 2^(k+1))), one jump per substream.  The
+ * jumps are queued on `stream`, which must not be capturing; use the pool
+ * there, or after it. */
 int mtgp32_gpu_pool_create_substreams(mtgp32_gpu_pool_t **out,
                                       const mtgp32_params_fast_t *para,
                                       uint32_t seed, int count,

@@ -1092,6 +1092,8 @@ struct Pool {
         // which a stream without its ordering does not wait
         CK(cudaStreamSynchronize(nullptr), "synchronize");
         CK(T::seed(d_params, d_pidx, nullptr, seed, d_states, 1, size, stride, S(s)), "seed");
+        // one stream is ready for any CUDA stream, as a seeded pool is
+        if (count == 1) CK(cudaStreamSynchronize(S(s)), "seed");
         // Doubling: level k makes windows [2^k, 2^(k+1)) from windows
         // [0, 2^k), each by one jump of X^(2^k * step) = table row k/2,
         // applied twice for odd k (the table holds the steps 4^r * step).

@@ -209,6 +209,7 @@ extern "C" {
                                              int count, const uint32_t *table, int rows,         \
                                              int nwords, void *s) {                              \
         int rc = newObj(out);                                                                    \
+        if (!rc) rc = notCapturing(s, "substreams");                                             \
         if (!rc) rc = (*out)->pool.init(p, 1, nullptr, count);                                   \
         if (!rc) rc = (*out)->pool.substreams(seed, table, rows, nwords, s);                     \
         if (rc && out && *out) {                                                                 \
