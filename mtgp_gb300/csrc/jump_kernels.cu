@@ -90,9 +90,14 @@ k_jump_part(const typename G::Tr::P *__restrict__ params, const typename G::W *_
 }
 
 // The longer exponents: the taps unsorted, against a ring that holds part of
-// the sequence (jump_device.cuh).  An early form of the sorted kernel did not
-// end at MEXP 44497, although the same code does when its threads are run on
-// the CPU; the cause is not known, so it stays off there.
+// the sequence (jump_device.cuh).  Early forms of the sorted kernel did not end
+// at MEXP 44497 (704 threads).  The first had the aligned barrier, without a
+// __syncwarp, behind loops that a warp's lanes left at different trips, which
+// is undefined; of the second, with the unaligned barrier, the cause is not
+// known.  The shapes that the sorted kernel is run with reach every barrier by
+// whole warps, each lane at the same trip (SJump, barN), in loops whose bounds
+// are the same for a barrier's whole group; MEXP 44497 and 110503 have not been
+// run with this form.
 template <class Tr, class Geo>
 __global__ void __launch_bounds__(Geo::NT)
 k_jump_ring(const typename Tr::P *__restrict__ params, typename Tr::W *__restrict__ states,

@@ -54,12 +54,18 @@ struct SJump {
     static constexpr int WARPS = CWARPS > GWARPS + 4 ? CWARPS : GWARPS + 4;
     static constexpr int NT = 32 * WARPS;
     static constexpr int ST = NT - GW;                         // threads that sort
-    static constexpr int ROWS = C / 8 + 260;  // each pattern's list even, four more behind
+    // each pattern's list even, four more behind, whole warps' loops over it
+    static constexpr int ROWS = (C / 8 + 260 + 31) & ~31;
     static constexpr int SEQ = C + PIECES * 128 / WS;          // words of the sequence buffer
     static constexpr int ZERO = SEQ * (int)sizeof(W);          // a row of zeros behind it
     static constexpr int NJ = (N + 3) & ~3;
     static_assert(C % 128 == 0 && GW % 32 == 0 && C >= N && C >= GW && NT <= 1024, "bad jump geometry");
     static_assert(SEQ >= C + N, "sequence buffer too small");
+    // barN's conditions: its groups are whole warps, one of them at least, and
+    // every loop before it runs over a multiple of 32 in steps of its group, so
+    // that no two lanes of a warp leave one at different trips
+    static_assert(ST % 32 == 0 && ST >= 32 && GW % 32 == 0 && ROWS % 32 == 0,
+                  "a warp would reach a barrier in parts");
     static constexpr size_t off_jout = ZERO + PIECES * 512;
     static constexpr size_t off_rows = off_jout + sizeof(W) * NJ;
     static constexpr size_t off_ends = off_rows + 4 * ROWS;
@@ -68,9 +74,12 @@ struct SJump {
     static_assert(kBytes <= 227 * 1024, "jump buffers exceed shared memory");
 };
 
-// Barrier `id` of `threads` threads, whole warps.
+// Barrier `id` of `threads` threads, whole warps.  The aligned form is undefined
+// unless a warp's lanes arrive as one: the loops before it end at the same trip
+// for all of them (SJump's static_assert), and __syncwarp brings them together
+// again behind the branches inside.
 __device__ __forceinline__ void barN(int id, int threads) {
-    __syncwarp();  // the loops before it end at different trips within a warp
+    __syncwarp();
     asm volatile("barrier.sync.aligned %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
