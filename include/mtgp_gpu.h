@@ -427,9 +427,9 @@ int mtgp_gpu_plan_describe(const mtgp_gpu_plan_t *plan, int64_t *values,
  * rule: do not change them while another thread plans with the handle.
  * Keys:
  *   "split_chunk"  0 = automatic, < 0 = never split, > 0 = chunk length
- *   "batch_grid"   CTAs of a plan's launch: 0 = automatic (four per SM, two at
- *                  MEXP 23209, every resident slot above), > 0 = that
- *                  many
+ *   "batch_grid"   CTAs of a plan's launch: 0 = automatic (every resident
+ *                  slot, or four per SM, two at MEXP 23209, where the longest
+ *                  tasks set the launch's length), > 0 = that many
  *   "core"         32-bit generation core: 2 = two adjacent words per
  *                  thread (default), 4 = four, 1 = one word per thread; plans
  *                  whose items mix output kinds use the one-word core

@@ -3,8 +3,8 @@
 //
 // A batch is a list of tasks; a task is one stream and a chain of work items
 // (count, output kind, output byte offset) that continue that stream in
-// order.  The grid is a few CTAs per SM (planCtas), or what the caller asks
-// for; a CTA's first task is its own number and it takes the next ones from a
+// order.  The grid is every resident CTA, a few per SM (fewCtas), or what the
+// caller asks for; a CTA's first task is its own number and it takes the next ones from a
 // device counter (tasks are sorted longest-first on the host, so the long ones
 // start first), loads the stream's window into shared memory, runs the items
 // with a generation core, and writes the advanced window back.

@@ -57,8 +57,8 @@ inline int notCapturing(void *s, const char *what) {
 
 // Tuning knobs (mtgp_gpu_set_tuning).  split_chunk: 0 = automatic, < 0 =
 // never split long requests, > 0 = split into chunks of this many values.
-// batch_grid: 0 = automatic (planCtas() CTAs per SM, or every resident slot
-// for the longer exponents), > 0 = that many CTAs.
+// batch_grid: 0 = automatic (every resident slot, or planCtas() CTAs per SM
+// where fewCtas says so), > 0 = that many CTAs.
 // A skip at least this long is done by a GF(2) jump inside the batched
 // kernel (about the work of 2^17 generated values) instead of generation.
 constexpr uint64_t kJumpMinSkip = 1 << 17;

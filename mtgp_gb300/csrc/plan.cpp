@@ -275,7 +275,9 @@ int makePlan(Pool<T> &P, const mtgp_work_item_t *items, int nitems, mtgp_gpu_pla
     pl->mode = mode;
     pl->out_bytes = out_bytes;
     pl->grid = (int)P.tune.batch_grid;
-    pl->auto_grid = few ? planCtas(P.sh.mexp) * P.pow_width : 0;
+    // (the four-word core's CTAs are half as wide: all that fit, 4096 x 65536
+    // values 259 us, 413 on four per SM)
+    pl->auto_grid = core != 4 && fewCtas(R, o) ? o.ctas * o.sms : 0;
     pl->split = split;
     pl->core = core;
     pl->chunk = cut ? chunk : 0;

@@ -59,12 +59,12 @@ struct PlanOptions {
     int sms = 0, ctas = 4, jump_values = 150;
 };
 
-// CTAs per SM of a plan's launch, where nothing else is asked for.
+// CTAs per SM of a plan's launch where long runs set its length (fewCtas).
 // Four of 11213's fill an SM's data pipe (4096
 // lognormal streams of 32-bit words: 429 us on four, 456 on three and five,
 // 625 on all ten that fit; 1024 streams of 64-bit words: 243 us, 264, 247,
-// 356), and the fewer share it the sooner the longest tasks end, which set
-// the length of a launch.  Two of 23209's, which have twice the threads (512
+// 356), and the fewer share it the sooner the longest tasks end.  Two of
+// 23209's, which have twice the threads (512
 // streams: 119 us on two, 144 on three, 168 on four).
 inline int planCtas(int mexp) { return mexp == 11213 ? 4 : 2; }
 
@@ -92,6 +92,27 @@ struct PlanResult {
     uint64_t out_bytes = 0;             // max over items of offset + size
     int mode = -1;                      // shared kind of all values, -1 all advance, -2 mixed
 };
+
+// Whether a plan runs on few CTAs per SM (planCtas) instead of all that fit.
+// Few pay where the longest tasks set the launch's length: these are long, the
+// tasks not so many that the work as a whole does, and the first of the second
+// round is short beside the longest (equal tasks just over a round would take
+// two).  Over 1150 plans of more tasks than few slots (to 10000 tasks; equal,
+// lognormal and other lengths; every core but the four-word one; both
+// exponents) few took 0.95 of the time of all (0.78 to 1.12) where this holds
+// and 1.21 (0.87 to 2.3) where it does not:
+//   4096 lognormal streams, median 65536     414 us on few, 428 on all
+//   640 of 1 to 131071 values, 64-bit 23209   81            102
+//   640 x 16384 (two rounds)                  24             19
+//   10000 x 1000 (short tasks)                52             33
+inline bool fewCtas(const PlanResult &r, const PlanOptions &o) {
+    const size_t slots = (size_t)o.ctas * (size_t)o.sms, n = r.tasks.size();
+    const size_t rounds = o.word_bytes == 8 ? 8 : 6;
+    if (slots == 0 || n == 0 || n > rounds * slots || r.tasks[0].total < o.jump_min / 2)
+        return false;
+    return n <= slots ||
+           5 * (r.tasks[slots - 1].total + r.tasks[slots].total) <= 7 * r.tasks[0].total;
+}
 
 // Returns MTGP_OK or an MTGP_ERR_* code with a message in *err.
 int planCore(const mtgp_work_item_t *items, int nitems, const PlanOptions &o, PlanResult *r,
