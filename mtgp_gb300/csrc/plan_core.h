@@ -99,7 +99,7 @@ struct PlanResult {
 // round is short beside the longest (equal tasks just over a round would take
 // two).  Over 1150 plans of more tasks than few slots (to 10000 tasks; equal,
 // lognormal and other lengths; every core but the four-word one; both
-// exponents) few took 0.95 of the time of all (0.78 to 1.12) where this holds
+// exponents) few took 0.96 of the time of all (0.78 to 1.23) where this holds
 // and 1.21 (0.87 to 2.3) where it does not:
 //   4096 lognormal streams, median 65536     414 us on few, 428 on all
 //   640 of 1 to 131071 values, 64-bit 23209   81            102
@@ -107,8 +107,7 @@ struct PlanResult {
 //   10000 x 1000 (short tasks)                52             33
 inline bool fewCtas(const PlanResult &r, const PlanOptions &o) {
     const size_t slots = (size_t)o.ctas * (size_t)o.sms, n = r.tasks.size();
-    const size_t rounds = o.word_bytes == 8 ? 8 : 6;
-    if (slots == 0 || n == 0 || n > rounds * slots || r.tasks[0].total < o.jump_min / 2)
+    if (slots == 0 || n == 0 || n > 8 * slots || r.tasks[0].total < o.jump_min / 2)
         return false;
     return n <= slots ||
            5 * (r.tasks[slots - 1].total + r.tasks[slots].total) <= 7 * r.tasks[0].total;
