@@ -126,15 +126,18 @@ constexpr int mixBlocks(int blocks, size_t smem) {
 }
 
 // Threads per SM that fix a one-word kernel's registers: 1280, 48 registers,
-// where that leaves five CTAs or more (plans take four; with 2048, 32 registers,
-// the tempering behind the recursion spilled: 4000 mixed requests 84 us, 80
-// with 1280), else 2048.
-constexpr int oneWordThreads(int tn, bool split) { return split || tn <= 256 ? 1280 : 2048; }
+// where that leaves five CTAs or more (deferring the outputs takes 44 to 48),
+// else 2048.  The mixed kernels take 2048, 32 registers, and do not defer:
+// their plans are many requests, for which eight CTAs per SM hide more (10000 x
+// 1000 values of three kinds 38 us, 44 deferred on five; 4096 x 16384 83, 93).
+constexpr int oneWordThreads(int tn, bool split, bool mixed) {
+    return split || (tn <= 256 && !mixed) ? 1280 : 2048;
+}
 
 template <int N, int TN, int B, int KIND>
 __device__ __noinline__ void mix32(Lane32 L, uint64_t n, char *o) {
     using OT = typename Out32<(KIND < 0 ? 0 : KIND)>::T;
-    run32<N, TN, B, KIND>(g_mix32, L, L.otab(KIND < 0 ? 0 : KIND), n, (OT *)o);
+    run32<N, TN, B, KIND, false>(g_mix32, L, L.otab(KIND < 0 ? 0 : KIND), n, (OT *)o);
 }
 
 template <int N, int W, int B, int KIND, int K>
@@ -146,7 +149,7 @@ __device__ __noinline__ void mixk32(Lane32 L, uint64_t n, char *o) {
 template <int N, int TN, int B, int KIND>
 __device__ __noinline__ void mix64(Lane64 L, uint64_t n, char *o) {
     using OT = typename Out64<(KIND < 0 ? 0 : KIND)>::T;
-    run64<N, TN, B, KIND>(g_mix64, L, L.otab_lo(KIND < 0 ? 0 : KIND),
+    run64<N, TN, B, KIND, false>(g_mix64, L, L.otab_lo(KIND < 0 ? 0 : KIND),
                           L.otab_hi(KIND < 0 ? 0 : KIND), n, (OT *)o);
 }
 
@@ -155,8 +158,8 @@ __device__ __noinline__ void mix64(Lane64 L, uint64_t n, char *o) {
 // B words).  SPLIT: tasks may start with a jump.
 template <int N, int TN, int B, int MODE, bool SPLIT>
 __global__ void __launch_bounds__(TN, MODE == -2
-                                         ? mixBlocks(oneWordThreads(TN, SPLIT) / TN, sizeof(uint32_t) * B)
-                                         : oneWordThreads(TN, SPLIT) / TN)
+                                         ? mixBlocks(oneWordThreads(TN, SPLIT, true) / TN, sizeof(uint32_t) * B)
+                                         : oneWordThreads(TN, SPLIT, false) / TN)
 k_batch32(const DevParams32 *__restrict__ params, uint32_t *__restrict__ states,
           const BatchTask *__restrict__ tasks, int ntasks,
           const BatchItem *__restrict__ items, char *__restrict__ out,
@@ -296,8 +299,8 @@ k_batch32xk(const DevParams32 *__restrict__ params, uint32_t *__restrict__ state
 
 template <int N, int TN, int B, int MODE, bool SPLIT>
 __global__ void __launch_bounds__(TN, MODE == -2
-                                         ? mixBlocks(oneWordThreads(TN, SPLIT) / TN, sizeof(uint64_t) * B)
-                                         : oneWordThreads(TN, SPLIT) / TN)
+                                         ? mixBlocks(oneWordThreads(TN, SPLIT, true) / TN, sizeof(uint64_t) * B)
+                                         : oneWordThreads(TN, SPLIT, false) / TN)
 k_batch64(const DevParams64 *__restrict__ params, uint64_t *__restrict__ states,
           const BatchTask *__restrict__ tasks, int ntasks,
           const BatchItem *__restrict__ items, char *__restrict__ out,

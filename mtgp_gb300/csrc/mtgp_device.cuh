@@ -213,27 +213,22 @@ __device__ __forceinline__ void compact(W *buf, uint32_t src) {
     __syncthreads();
 }
 
-// One sub-step for 32-bit words, px = buf + base + t, py = px + pos: the word
-// made (r) and the one that tempers it (t).  `meanwhile`, the outputs of the
-// sub-step before, runs behind the shared store (CoreK::sub says why).
+// One sub-step for 32-bit words, px = buf + base + t, py = px + pos.  `out` gets
+// the word made and the one that tempers it, behind the shared store.
 template <int N, class F>
-__device__ __forceinline__ void sub32(uint32_t *px, const Lane32 &L, uint32_t mul1, uint32_t &r,
-                                      uint32_t &t, F meanwhile) {
+__device__ __forceinline__ void sub32(uint32_t *px, const Lane32 &L, uint32_t mul1, F out) {
     const uint32_t *py = px + L.pos;
     const uint32_t x1 = px[0], x2 = px[1], y = py[0], tt = py[-1];
     const uint32_t x = (x1 & L.mask) ^ x2;
     const uint32_t yy = x ^ (x * mul1) ^ (y >> L.sh2);
     const uint32_t v = yy ^ lut(L.tbl, yy);
     px[N] = v;
-    meanwhile();
-    r = v;
-    t = tt;
+    out(v, tt);
     __syncthreads();
 }
 
 template <int N, class F>
-__device__ __forceinline__ void sub64(uint64_t *px, const Lane64 &L, uint32_t mul1, uint64_t &r,
-                                      uint32_t &t, F meanwhile) {
+__device__ __forceinline__ void sub64(uint64_t *px, const Lane64 &L, uint32_t mul1, F out) {
     const uint64_t *py = px + L.pos;
     const uint64_t x1 = px[0], x2 = px[1], y = py[0], tt = py[-1];
     const uint64_t x = (x1 & L.mask) ^ x2;
@@ -245,15 +240,15 @@ __device__ __forceinline__ void sub64(uint64_t *px, const Lane64 &L, uint32_t mu
     yl = xh ^ (yl >> L.sh2);
     const uint64_t v = (((uint64_t)yh << 32) | yl) ^ lut64(L.tbl_lo, L.tbl_hi, yl);
     px[N] = v;
-    meanwhile();
-    r = v;
-    t = (uint32_t)tt;
+    out(v, (uint32_t)tt);
     __syncthreads();
 }
 
 // Advance by n steps writing n outputs of KIND (KIND < 0: no output).
-// otab*: lane value of the output table (Lane32::otab(KIND)).
-template <int N, int TN, int B, int KIND>
+// otab*: lane value of the output table (Lane32::otab(KIND)).  DEFER: a
+// sub-step's outputs are written while the next one waits (CoreK::sub says
+// why), but not in the last, partial segment (GeoK::kLongTail says why).
+template <int N, int TN, int B, int KIND, bool DEFER = true>
 __device__ __forceinline__ void run32(uint32_t *buf, const Lane32 &L, uint32_t otab,
                                       uint64_t n,
                                       typename Out32<(KIND < 0 ? 0 : KIND)>::T *out) {
@@ -263,19 +258,25 @@ __device__ __forceinline__ void run32(uint32_t *buf, const Lane32 &L, uint32_t o
     uint32_t *px = buf + t;
     auto *o = out + t;
     uint32_t pr, pt;  // of the sub-step not yet written out
-    auto emit = [&](auto *to, bool live) {
+    auto emit = [&](auto r, uint32_t tt, auto *to, bool live) {
         if constexpr (KIND >= 0) {
-            const uint32_t ov = lut(otab, fold(pt));
-            if (live) *to = Out32<KIND>::conv(pr, ov);
+            const uint32_t ov = lut(otab, fold(tt));
+            if (live) *to = Out32<KIND>::conv(r, ov);
         }
     };
     while (n >= (uint64_t)S * TN) {
 #pragma unroll
         for (int k = 0; k < S; k++)
-            sub32<N>(px + k * TN, L, mul1, pr, pt, [&] {
-                if (k > 0) emit(o + (k - 1) * TN, true);
+            sub32<N>(px + k * TN, L, mul1, [&](auto r, uint32_t tt) {
+                if constexpr (DEFER) {
+                    if (k > 0) emit(pr, pt, o + (k - 1) * TN, true);
+                    pr = r;
+                    pt = tt;
+                } else {
+                    emit(r, tt, o + k * TN, true);
+                }
             });
-        emit(o + (S - 1) * TN, true);
+        if constexpr (DEFER) emit(pr, pt, o + (S - 1) * TN, true);
         compact<uint32_t, N, TN>(buf, S * TN);
         n -= (uint64_t)S * TN;
         if constexpr (KIND >= 0) o += S * TN;
@@ -284,14 +285,12 @@ __device__ __forceinline__ void run32(uint32_t *buf, const Lane32 &L, uint32_t o
     if (rem == 0) return;
     const int subs = (rem + TN - 1) / TN;
     for (int k = 0; k < subs; k++)
-        sub32<N>(px + k * TN, L, mul1, pr, pt, [&] {
-            if (k > 0) emit(o + (k - 1) * TN, true);
-        });
-    emit(o + (subs - 1) * TN, (subs - 1) * TN + t < rem);
+        sub32<N>(px + k * TN, L, mul1,
+                 [&](auto r, uint32_t tt) { emit(r, tt, o + k * TN, k * TN + t < rem); });
     compact<uint32_t, N, TN>(buf, (uint32_t)rem);
 }
 
-template <int N, int TN, int B, int KIND>
+template <int N, int TN, int B, int KIND, bool DEFER = true>
 __device__ __forceinline__ void run64(uint64_t *buf, const Lane64 &L, uint32_t olo,
                                       uint32_t ohi, uint64_t n,
                                       typename Out64<(KIND < 0 ? 0 : KIND)>::T *out) {
@@ -302,19 +301,25 @@ __device__ __forceinline__ void run64(uint64_t *buf, const Lane64 &L, uint32_t o
     auto *o = out + t;
     uint64_t pr;  // of the sub-step not yet written out
     uint32_t pt;
-    auto emit = [&](auto *to, bool live) {
+    auto emit = [&](auto r, uint32_t tt, auto *to, bool live) {
         if constexpr (KIND >= 0) {
-            const uint64_t ov = lut64(olo, ohi, fold(pt));
-            if (live) *to = Out64<KIND>::conv(pr, ov);
+            const uint64_t ov = lut64(olo, ohi, fold(tt));
+            if (live) *to = Out64<KIND>::conv(r, ov);
         }
     };
     while (n >= (uint64_t)S * TN) {
 #pragma unroll
         for (int k = 0; k < S; k++)
-            sub64<N>(px + k * TN, L, mul1, pr, pt, [&] {
-                if (k > 0) emit(o + (k - 1) * TN, true);
+            sub64<N>(px + k * TN, L, mul1, [&](auto r, uint32_t tt) {
+                if constexpr (DEFER) {
+                    if (k > 0) emit(pr, pt, o + (k - 1) * TN, true);
+                    pr = r;
+                    pt = tt;
+                } else {
+                    emit(r, tt, o + k * TN, true);
+                }
             });
-        emit(o + (S - 1) * TN, true);
+        if constexpr (DEFER) emit(pr, pt, o + (S - 1) * TN, true);
         compact<uint64_t, N, TN>(buf, S * TN);
         n -= (uint64_t)S * TN;
         if constexpr (KIND >= 0) o += S * TN;
@@ -323,10 +328,8 @@ __device__ __forceinline__ void run64(uint64_t *buf, const Lane64 &L, uint32_t o
     if (rem == 0) return;
     const int subs = (rem + TN - 1) / TN;
     for (int k = 0; k < subs; k++)
-        sub64<N>(px + k * TN, L, mul1, pr, pt, [&] {
-            if (k > 0) emit(o + (k - 1) * TN, true);
-        });
-    emit(o + (subs - 1) * TN, (subs - 1) * TN + t < rem);
+        sub64<N>(px + k * TN, L, mul1,
+                 [&](auto r, uint32_t tt) { emit(r, tt, o + k * TN, k * TN + t < rem); });
     compact<uint64_t, N, TN>(buf, (uint32_t)rem);
 }
 
