@@ -6,6 +6,7 @@
 // writes the advanced window back.  Unlike the sample it accepts any n (not
 // a multiple of 3*TN), any parameter set per CTA, all five output kinds and
 // every Mersenne exponent of the reference's tables.
+#include "cta_team.cuh"
 #include "mtgp_device64x2.cuh"
 
 namespace mtgp {
@@ -142,11 +143,21 @@ static cudaError_t gen64x2(int kind, const DevParams64 *params, const int *pidx,
     return cudaGetLastError();
 }
 
-// Values per generator from which the two-word kernels take the long buffer:
-// one and a half of its segments.  Five CTAs an SM still fit, more than its
-// data pipe needs; shorter fills are over before a window moves twice, and
-// keep the ten CTAs of the short one.
+// Whether a fill by the two-word kernels takes the long buffer: for 16384 values
+// (one and a half of its segments, six of the 64-bit one's) and more, where a
+// few generators have an SM, whose chains it shortens (456 x 65536 values 33 us,
+// 38 with the short one).  Five of its CTAs fit an SM, of the short one's ten:
+// more generators fill the data pipe either way, and those beyond a round of
+// five wait for it to end (912 x 20000 values 28 us, 24 with the short one; 4096
+// x 16384 74, 68).  64-bit words: nine fit an SM, of the short one's thirteen,
+// which run no faster than nine (2000 x 65536 values 266 us, 244 with the long
+// one; 1520, a round of ten on the short one, 176 and 184).
 constexpr uint64_t kLongFill = 16384;
+static bool longFill(uint64_t n, int ngen, size_t word) {
+    if (n < kLongFill) return false;
+    const int sms = smCount();
+    return ngen <= 4 * sms || (word == 8 && ngen >= 12 * sms);
+}
 
 template <int N, int TN, int B>
 static cudaError_t gen32_kind(int kind, const DevParams32 *params, const int *pidx,
@@ -154,7 +165,7 @@ static cudaError_t gen32_kind(int kind, const DevParams32 *params, const int *pi
                               uint64_t os, cudaStream_t s, int core) {
     dim3 grid(ngen), block(TN);
     if (core == 4) return gen32xk<N, TN, B, 4>(kind, params, pidx, states, ngen, out, n, os, s);
-    if (core != 1 && n >= kLongFill)
+    if (core != 1 && longFill(n, ngen, 4))
         return gen32xk<N, TN, kLongBuf<N, B>, 2>(kind, params, pidx, states, ngen, out, n, os, s);
     if (core != 1) return gen32xk<N, TN, B, 2>(kind, params, pidx, states, ngen, out, n, os, s);
     switch (kind) {
@@ -174,7 +185,7 @@ static cudaError_t gen64_kind(int kind, const DevParams64 *params, const int *pi
                               uint64_t *states, int ngen, void *out, uint64_t n,
                               uint64_t os, cudaStream_t s, int core) {
     dim3 grid(ngen), block(TN);
-    if (core != 1 && n >= kLongFill)
+    if (core != 1 && longFill(n, ngen, 8))
         return gen64x2<N, TN, kLongBuf<N, B>>(kind, params, pidx, states, ngen, out, n, os, s);
     if (core != 1) return gen64x2<N, TN, B>(kind, params, pidx, states, ngen, out, n, os, s);
     switch (kind) {
