@@ -64,12 +64,15 @@ int makePlan(Pool<T> &P, const mtgp_work_item_t *items, int nitems, mtgp_gpu_pla
     o.resident = o.can_jump ? T::resident(P.sh.mexp, P.tune.jump_parts < 0, core) : 1;
     // MEXP 11213 and 23209 with jumps made ahead of the launch: few CTAs per
     // SM and the chunk that goes with them (the longer exponents' CTAs are up
-    // to 1024 threads, and few fit an SM).  A jump costs about mexp^2.
+    // to 1024 threads, and few fit an SM).  A jump costs about mexp^2; a value
+    // of 32-bit 23209 takes half as long, so their launch costs more of them (64
+    // lognormal streams: 40 us with three jumps, 31 uncut).
     const bool few = T::splits(P.sh.mexp) && P.tune.jump_parts >= 0;
     if (few) {
         o.sms = P.pow_width;
         o.ctas = planCtas(P.sh.mexp);
         o.jump_values = P.sh.mexp == 11213 ? 150 : 1250;
+        o.jump_launch = P.sh.mexp == 23209 && T::kBits == 32 ? 70000 : 17000;
     }
     // scratch reused by every plan made on this thread
     static thread_local PlanResult R;

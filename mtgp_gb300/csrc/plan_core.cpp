@@ -59,16 +59,22 @@ uint64_t cutRun(uint64_t total, uint64_t chunk, uint64_t grain, uint64_t *piece)
 // 0.42 with three, 0.30 with one or two, 32-bit; 1.0 ns with three or four and
 // 0.75 with fewer, 64-bit):
 //   - the jumps, one per piece but a run's first: o.jump_values each (85 and
-//     107 ns on the whole GPU) after the 17 k that the launch before takes;
+//     107 ns on the whole GPU) after the o.jump_launch that the launch before
+//     takes;
 //   - the generation: the CTAs' even share of the values, or the long pieces
 //     (over half of the longest) in the rounds that the CTAs need for them,
-//     whichever is longer; the short ones fill what is left.
-// Over 14 workloads (16 to 4096 streams, lognormal and equal lengths, both
-// word sizes) the choice was within 7 % of the best of 15 lengths.  Where no
+//     whichever is longer; the short ones fill what is left;
+//   - with the grid of all resident CTAs (fewCtas): uncut runs that fit it at
+//     once share an SM by that many, and of more tasks than few CTAs are for,
+//     what is left of the longest one behind the even share runs nearly alone.
+// Over 366 plans (1 to 10000 streams, lognormal, even and equal lengths, one
+// kind and three, both word sizes, MEXP 11213 and 23209) the launch took 1.03
+// of the time with the best of 12 lengths on average, 1.33 at most (1.04 and
+// 1.37 without the last item, which 400 x 2^20 values at MEXP 23209 showed: 573
+// us cut in two, 418 uncut).  Where no
 // run is longer than jump_min nothing is cut: a pool without jumps needs no
 // jump tables, which take longer to make than such a launch.
 int64_t cheapestChunk(const std::vector<Run> &runs, uint64_t grand, const PlanOptions &o) {
-    constexpr double kJumps = 17000;
     constexpr uint64_t kShortest = uint64_t(1) << 15;
     thread_local std::vector<uint64_t> longs;
     longs.clear();
@@ -105,9 +111,16 @@ int64_t cheapestChunk(const std::vector<Run> &runs, uint64_t grand, const PlanOp
             const double slow = std::min(1.0, o.word_bytes == 4 ? std::max(0.5, (double)per_sm / o.ctas)
                                               : 2 * per_sm <= (uint64_t)o.ctas ? 0.75 : 1.0);
             const uint64_t rounds = (nbig + slots - 1) / slots;
-            const double gen = std::max(share, rounds <= 1 ? slow * (double)top
-                                                           : (double)rounds * big / (double)nbig);
-            const double cost = gen + (double)o.jump_values * (double)jumps + (jumps ? kJumps : 0);
+            double gen = std::max(share, rounds <= 1 ? slow * (double)top
+                                                     : (double)rounds * big / (double)nbig);
+            if (tasks > kFewRounds * slots) {
+                const double rate = (double)slots / (double)std::max<uint64_t>(o.resident, slots);
+                gen = share + std::max(0.0, (double)top - rate * share) / 2;
+            } else if (jumps == 0 && rounds > 1 && tasks <= (uint64_t)o.resident) {
+                gen = std::max(share, (double)top * (double)per_sm / o.ctas);
+            }
+            const double cost = gen + (double)o.jump_values * (double)jumps +
+                                (jumps ? (double)o.jump_launch : 0);
             if (!best || cost <= best_cost) {
                 best = (int64_t)chunk;
                 best_cost = cost;

@@ -55,8 +55,9 @@ struct PlanOptions {
     // > 0: SMs of the GPU, for plans whose jumps are made ahead of the launch
     // and whose grid is `ctas` CTAs per SM; the automatic chunk is then the
     // cheapest (cheapestChunk), not a power of two.  jump_values: what a jump
-    // costs, in values generated by one CTA
-    int sms = 0, ctas = 4, jump_values = 150;
+    // costs, in values generated by one CTA; jump_launch: what the launch of
+    // any number of them does
+    int sms = 0, ctas = 4, jump_values = 150, jump_launch = 17000;
 };
 
 // CTAs per SM of a plan's launch where long runs set its length (fewCtas).
@@ -105,9 +106,10 @@ struct PlanResult {
 //   640 of 1 to 131071 values, 64-bit 23209   81            102
 //   640 x 16384 (two rounds)                  24             19
 //   10000 x 1000 (short tasks)                52             33
+constexpr size_t kFewRounds = 8;
 inline bool fewCtas(const PlanResult &r, const PlanOptions &o) {
     const size_t slots = (size_t)o.ctas * (size_t)o.sms, n = r.tasks.size();
-    if (slots == 0 || n == 0 || n > 8 * slots || r.tasks[0].total < o.jump_min / 2)
+    if (slots == 0 || n == 0 || n > kFewRounds * slots || r.tasks[0].total < o.jump_min / 2)
         return false;
     return n <= slots ||
            5 * (r.tasks[slots - 1].total + r.tasks[slots].total) <= 7 * r.tasks[0].total;
