@@ -76,7 +76,11 @@ uint64_t cutRun(uint64_t total, uint64_t chunk, uint64_t grain, uint64_t *piece)
 // jump tables, which take longer to make than such a launch.
 int64_t cheapestChunk(const std::vector<Run> &runs, uint64_t grand, const PlanOptions &o) {
     constexpr uint64_t kShortest = uint64_t(1) << 15;
+    struct Cut {
+        uint64_t k, piece, rest;
+    };
     thread_local std::vector<uint64_t> longs;
+    thread_local std::vector<Cut> cuts;
     longs.clear();
     uint64_t longest = 0;
     for (const Run &R : runs) {
@@ -86,47 +90,56 @@ int64_t cheapestChunk(const std::vector<Run> &runs, uint64_t grand, const PlanOp
     if (longest <= o.jump_min) return (int64_t)o.jump_min;
     const uint64_t slots = (uint64_t)o.ctas * (uint64_t)o.sms;
     const double share = (double)grand / (double)slots;
+    // 4, 5, 6 and 7 times a power of two, from one above twice the even share
+    // or one that cuts nothing down, until the jumps alone cost too much
+    uint64_t base = kShortest / 4, m = 4;
+    while (m * base < longest && (double)(m * base) <= 2 * share + (double)o.jump_min)
+        if (++m == 8) base *= 2, m = 4;
     int64_t best = 0;
     double best_cost = 0;
-    // 4, 5, 6 and 7 times a power of two, up to twice the even share or one
-    // that cuts nothing
-    for (uint64_t base = kShortest / 4;; base *= 2) {
-        for (uint64_t m = 4; m < 8; m++) {
-            const uint64_t chunk = m * base, grain = cheapGrain(chunk);
-            uint64_t jumps = 0, top = 0, piece = 0;
-            for (uint64_t t : longs) {
-                jumps += cutRun(t, chunk, grain, &piece) - 1;
-                top = std::max(top, piece);
-            }
-            uint64_t nbig = 0;
-            double big = 0;
-            for (uint64_t t : longs) {
+    for (;;) {
+        const uint64_t chunk = m * base, grain = cheapGrain(chunk);
+        uint64_t jumps = 0, top = 0;
+        cuts.clear();
+        for (uint64_t t : longs) {
+            uint64_t piece = t;
+            if (t > chunk) {
                 const uint64_t k = cutRun(t, chunk, grain, &piece);
-                const uint64_t rest = t - (k - 1) * piece;
-                if (2 * piece > top) nbig += k - 1, big += (double)((k - 1) * piece);
-                if (2 * rest > top) nbig++, big += (double)rest;
+                cuts.push_back({k, piece, t - (k - 1) * piece});
+                jumps += k - 1;
             }
-            const uint64_t tasks = runs.size() + jumps;
-            const uint64_t per_sm = (tasks + (uint64_t)o.sms - 1) / (uint64_t)o.sms;
-            const double slow = std::min(1.0, o.word_bytes == 4 ? std::max(0.5, (double)per_sm / o.ctas)
-                                              : 2 * per_sm <= (uint64_t)o.ctas ? 0.75 : 1.0);
-            const uint64_t rounds = (nbig + slots - 1) / slots;
-            double gen = std::max(share, rounds <= 1 ? slow * (double)top
-                                                     : (double)rounds * big / (double)nbig);
-            if (tasks > kFewRounds * slots) {
-                const double rate = (double)slots / (double)std::max<uint64_t>(o.resident, slots);
-                gen = share + std::max(0.0, (double)top - rate * share) / 2;
-            } else if (jumps == 0 && rounds > 1 && tasks <= (uint64_t)o.resident) {
-                gen = std::max(share, (double)top * (double)per_sm / o.ctas);
-            }
-            const double cost = gen + (double)o.jump_values * (double)jumps +
-                                (jumps ? (double)o.jump_launch : 0);
-            if (!best || cost <= best_cost) {
-                best = (int64_t)chunk;
-                best_cost = cost;
-            }
-            if (jumps == 0 || (double)chunk > 2 * share + (double)o.jump_min) return best;
+            top = std::max(top, piece);
         }
+        const double jump_cost = (double)o.jump_values * (double)jumps +
+                                 (jumps ? (double)o.jump_launch : 0);
+        if (best && share + jump_cost > best_cost) return best;
+        uint64_t nbig = 0;
+        double big = 0;
+        for (uint64_t t : longs)
+            if (t <= chunk && 2 * t > top) nbig++, big += (double)t;
+        for (const Cut &c : cuts) {
+            if (2 * c.piece > top) nbig += c.k - 1, big += (double)((c.k - 1) * c.piece);
+            if (2 * c.rest > top) nbig++, big += (double)c.rest;
+        }
+        const uint64_t tasks = runs.size() + jumps;
+        const uint64_t per_sm = (tasks + (uint64_t)o.sms - 1) / (uint64_t)o.sms;
+        const double slow = std::min(1.0, o.word_bytes == 4 ? std::max(0.5, (double)per_sm / o.ctas)
+                                          : 2 * per_sm <= (uint64_t)o.ctas ? 0.75 : 1.0);
+        const uint64_t rounds = (nbig + slots - 1) / slots;
+        double gen = std::max(share, rounds <= 1 ? slow * (double)top
+                                                 : (double)rounds * big / (double)nbig);
+        if (tasks > kFewRounds * slots) {
+            const double rate = (double)slots / (double)std::max<uint64_t>(o.resident, slots);
+            gen = share + std::max(0.0, (double)top - rate * share) / 2;
+        } else if (jumps == 0 && rounds > 1 && tasks <= (uint64_t)o.resident) {
+            gen = std::max(share, (double)top * (double)per_sm / o.ctas);
+        }
+        if (!best || gen + jump_cost < best_cost) {
+            best = (int64_t)chunk;
+            best_cost = gen + jump_cost;
+        }
+        if (chunk == kShortest) return best;
+        if (m-- == 4) base /= 2, m = 7;
     }
 }
 
