@@ -281,6 +281,9 @@ constexpr size_t kPowSmemPair = 113 * 1024;  // two CTAs per SM
 }  // namespace
 
 bool powOpsFits(int W) { return W > 0 && powSmemWords<2>(W, 1) * 4 <= kPowSmemMax; }
+bool powOpsWide(int W, int window) {
+    return window != 2 && powSmemWords<4>(W, 1) * 4 <= kPowSmemMax;
+}
 
 cudaError_t launchMonomials(uint32_t *blk, size_t tw, int W, int n, int i0, cudaStream_t s) {
     if (n <= 0 || i0 <= 0) return cudaSuccess;
@@ -299,7 +302,7 @@ static cudaError_t powOps(const PowOp *ops, const FewOps &few, bool chains, int 
                           const uint32_t *scratch, int W, cudaStream_t s, int window) {
     if (n <= 0) return cudaSuccess;
     if (!powOpsFits(W)) return cudaErrorInvalidValue;
-    const bool wide = window != 2 && powSmemWords<4>(W, 1) * 4 <= kPowSmemMax;
+    const bool wide = powOpsWide(W, window);
     const int sms = smCount();
     // more steps than SMs: two CTAs per SM (MEXP 11213, whose three tables fit
     // twice; 1000 chains of seven products take 2.01 ms, 2.38 with one CTA);

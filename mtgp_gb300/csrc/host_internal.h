@@ -945,10 +945,11 @@ struct Pool {
         if (rc) return rc;
         const int W = polyWords();
         PowSchedule sch;
-        if (n <= kFewOps) {
+        if (n <= kFewOps && powOpsWide(W, tune.poly_window)) {
             // a chain each, in one launch without upload or scratch: for one
             // exponent the tree's allocation alone took longer than its four
-            // more products in turn
+            // more products in turn (on clusters; at MEXP 110503, where a
+            // product is one CTA's 6.5 ms, a chain takes 39 ms, the tree 20)
             powSchedule(steps, n, 1, sch);
             std::vector<PowOp> ops;
             powOps(sch, [t](int) { return t; }, out, nullptr, sh.mexp, ops);

@@ -162,6 +162,9 @@ cudaError_t launchBarrett(const uint32_t *chi, int D, int n, int nw, size_t stri
                           cudaStream_t s);
 
 bool powOpsFits(int W);
+// Whether few products run on a cluster of CTAs each (launchPowOps): where the
+// table of the wider window fits in shared memory.
+bool powOpsWide(int W, int window);
 // Jump tables of n sets, tw words apart: the monomial slots X^(2^i), i <
 // i0; and a copy of the 64 slots X^(2^i) of each set into out (64 W words
 // per set).

@@ -208,6 +208,7 @@ bool shape64(int mexp, Shape *s) {
     return false;
 }
 bool powOpsFits(int W) { return W > 0; }
+bool powOpsWide(int W, int window) { return window != 2 && W < 3000; }
 bool batchSplits32(int mexp) { return mexp == 11213 || mexp == 23209; }
 bool batchSplits64(int mexp) { return mexp == 11213 || mexp == 23209; }
 int batchResident32(int, bool, int) { return 1520; }
