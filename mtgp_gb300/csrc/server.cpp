@@ -167,19 +167,22 @@ class DeviceRanges {
     explicit DeviceRanges(int device) : device_(device) {}
     bool holds(const void *p, uint64_t bytes) {
         const uint64_t a = reinterpret_cast<uint64_t>(p);
-        for (const auto &r : known_)
-            if (a >= r.first && a - r.first < r.second) return bytes <= r.second - (a - r.first);
+        if (const uint64_t left = known_.left(a)) return bytes <= left;
+        if (a >> kBlock == other_) return false;
         cudaPointerAttributes at;
         if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
             cudaGetLastError();
             return false;
         }
-        if (at.type != cudaMemoryTypeDevice || at.device != device_) return false;
+        if (at.type != cudaMemoryTypeDevice || at.device != device_) {
+            other_ = a >> kBlock;
+            return false;
+        }
         unsigned long long base = 0;
         size_t size = 0;
         const RangeFn fn = rangeFn();
         if (!fn || fn(&base, &size, a) != 0 || a < base || a - base >= size) return false;
-        known_.emplace_back(base, size);
+        known_.add(base, size);
         return bytes <= size - (a - base);
     }
 
@@ -198,7 +201,12 @@ class DeviceRanges {
         return fn;
     }
     int device_;
-    std::vector<std::pair<uint64_t, uint64_t>> known_;  // base, size
+    mtgp::RangeMap known_;
+    // The 2 MB of addresses where memory of another kind was found last: its
+    // neighbours are not asked for (a copy serves any kind).  4000 results to
+    // one pinned buffer 7.05 ms asking for each, 6.6 so.
+    static constexpr int kBlock = 21;
+    uint64_t other_ = ~uint64_t(0);
 };
 
 // Mark the requests whose values the kernel writes at their destination: in

@@ -66,6 +66,28 @@ class Arena {
     std::map<uint64_t, uint64_t> free_;  // offset -> length of each free block
 };
 
+// Ranges of memory that do not overlap, by address: the latest one found is
+// tried first (the requests of one buffer), then the others by a search.
+class RangeMap {
+  public:
+    // The range that holds address a: bytes from a to its end, 0 if none does.
+    uint64_t left(uint64_t a) {
+        if (a - base_ < size_) return size_ - (a - base_);
+        auto it = ranges_.upper_bound(a);
+        if (it == ranges_.begin()) return 0;
+        --it;
+        if (a - it->first >= it->second) return 0;
+        base_ = it->first;
+        size_ = it->second;
+        return size_ - (a - base_);
+    }
+    void add(uint64_t base, uint64_t size) { ranges_[base] = size; }
+
+  private:
+    std::map<uint64_t, uint64_t> ranges_;  // base -> size
+    uint64_t base_ = 0, size_ = 0;
+};
+
 struct ServeReq {
     uint64_t ticket;
     int pool;
