@@ -380,9 +380,9 @@ int mtgp64_gpu_pool_set_windows_host(mtgp64_gpu_pool_t *p,
 int mtgp64_gpu_pool_export(mtgp64_gpu_pool_t *p, int s, mtgp64_fast_t *dst);
 
 /* Autotuner (no reference counterpart): builds a plan for each candidate
- * configuration -- generation core (four words per thread in 64-thread CTAs
- * with 128-bit stores, or one word per thread in 256-thread CTAs), the chunk
- * length used to split long requests, and the grid size -- times each on
+ * configuration -- generation core (two, four or one words per thread), the
+ * chunk length used to split long requests, and the grid size; the pool's own
+ * choice of the last two with each core among them -- times each on
  * these items and this output buffer (median of `reps` launches on `stream`),
  * and returns the fastest.  The pool's windows are restored before every
  * trial and at the end, so the pool is left unchanged.  `report` (optional)
@@ -407,8 +407,8 @@ uint64_t mtgp_gpu_plan_output_bytes(const mtgp_gpu_plan_t *plan);
 int mtgp_gpu_plan_info(const mtgp_gpu_plan_t *plan, int64_t *tasks,
                        int64_t *chunk);
 /* The plan's configuration, the first n of: [0] tasks, [1] split chunk
- * length (0 = none), [2] generation core (1, 2 or 4), [3] grid (0 = all
- * resident CTAs), [4] kernels one launch runs, [5] 1 if tasks start with
+ * length (0 = none), [2] generation core (1, 2 or 4), [3] grid (0 =
+ * automatic, "batch_grid"), [4] kernels one launch runs, [5] 1 if tasks start with
  * in-kernel jumps, [6] tasks that start from a window jumped ahead of the
  * launch (by jump parts, before the persistent kernel), [7] 1 if those
  * tasks run in a second launch beside the first ("jump_overlap").  Passing

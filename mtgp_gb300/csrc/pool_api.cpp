@@ -9,11 +9,11 @@ namespace {
 // median of `reps` launches after one warm-up), and keep the fastest.  The
 // stream windows are restored from a snapshot before every launch, so every
 // candidate does exactly the same work and the pool ends where it started.
-// Candidates: generation core (32-bit: four words per thread in 64-thread
-// CTAs with 128-bit stores, or one word per thread in 256-thread CTAs with
-// 32-bit stores), split-chunk length for long requests (none, or 2^17 to
-// 2^20 in steps of 2^17, with either core), and grid size (all resident
-// CTAs, or 7/8, 3/4, 5/8, 1/2 of them).
+// Candidates: what the pool does by itself (its chunk length and grid), with
+// each generation core (32-bit: two words per thread, four, or one; 64-bit: two
+// or one), and with each core the split-chunk lengths none and 2^17 to 2^20 in
+// steps of 2^17 (2^17: the shortest jumped piece) on the automatic grid and on
+// all, 7/8, 3/4, 5/8, 1/2 and 3/8 of the resident CTAs.
 template <class T>
 int autotune(Pool<T> &P, const mtgp_work_item_t *items, int nitems, void *out, void *s,
              int reps, mtgp_gpu_plan **best, char *report, int cap) {
@@ -23,15 +23,14 @@ int autotune(Pool<T> &P, const mtgp_work_item_t *items, int nitems, void *out, v
     if (reps < 1) reps = 1;
     struct Cand {
         int core;
-        int64_t chunk, grid;
-        int overlap;
+        int64_t chunk;
     };
     std::vector<Cand> cands;
-    // 32-bit: four, two or one words per thread; 64-bit: two or one
-    const int cores32[3] = {4, 2, 1}, cores64[2] = {2, 1};
+    const int cores32[3] = {2, 4, 1}, cores64[2] = {2, 1};
     const int *cores = T::kBits == 32 ? cores32 : cores64;
     const int ncores = T::kBits == 32 ? 3 : 2;
-    for (int c = 0; c < ncores; c++) cands.push_back({cores[c], -1, 0, 0});
+    for (int c = 0; c < ncores; c++) cands.push_back({cores[c], 0});
+    for (int c = 0; c < ncores; c++) cands.push_back({cores[c], -1});
     // chunk lengths: 1..8 times the shortest jumped piece (2^17 at MEXP
     // 11213 and 23209)
     const int64_t base = std::max<int64_t>(int64_t(1) << 17, (int64_t)jumpMinSkip(P));
@@ -40,7 +39,7 @@ int autotune(Pool<T> &P, const mtgp_work_item_t *items, int nitems, void *out, v
     if (planJumps(P))
         for (int c = 0; c < ncores; c++)
             for (int64_t ch = base; ch <= 8 * base; ch += base)
-                cands.push_back({cores[c], ch, 0, 0});
+                cands.push_back({cores[c], ch});
     const size_t sbytes = sizeof(W) * (size_t)P.stride * P.count;
     W *snap = nullptr;
     CK(devMalloc(&snap, sbytes), "devMalloc(autotune snapshot)");
@@ -76,25 +75,29 @@ int autotune(Pool<T> &P, const mtgp_work_item_t *items, int nitems, void *out, v
         return MTGP_OK;
     };
     for (size_t k = 0; k < cands.size() && !rc; k++) {
-        static const int kGridEighths[] = {8, 7, 6, 5, 4, 3};  // of the resident CTAs
-        for (int g = 0; g < 6 && !rc; g++) {
+        static const int kGridEighths[] = {0, 8, 7, 6, 5, 4, 3};  // of the resident CTAs; 0 = automatic
+        static const char *const kGridNames[] = {"auto", "all", "7/8", "3/4", "5/8", "1/2", "3/8"};
+        for (int g = 0; g < (cands[k].chunk == 0 ? 1 : 7) && !rc; g++) {
             P.tune.split_chunk = cands[k].chunk;
             P.tune.batch_grid = 0;
             P.tune.core = cands[k].core;
-            P.tune.jump_overlap = cands[k].overlap;
+            P.tune.jump_overlap = 0;
             mtgp_gpu_plan *pl = nullptr;
             rc = makePlan(P, items, nitems, &pl);
             if (rc) break;
-            if ((cands[k].chunk > 0 && pl->chunk == 0) ||       // nothing long enough to split
-                (cands[k].overlap && !pl->overlap)) {           // nothing jumped ahead
+            if (cands[k].chunk > 0 && pl->chunk == 0) {  // nothing long enough to split
                 delete pl;
                 break;
+            }
+            if (g == 0 && cands[k].chunk != 0 && pl->auto_grid == 0) {  // "all" below
+                delete pl;
+                continue;
             }
             // fewer CTAs than resident: fewer share an SM's data pipe, so each
             // runs its tasks faster, which pays when the longest tasks set
             // the launch's length
             const int full = T::resident(P.sh.mexp, pl->split, pl->core);
-            pl->grid = std::max(1, full * kGridEighths[g] / 8);
+            if (g > 0) pl->grid = std::max(1, full * kGridEighths[g] / 8);
             float ms = 0;
             rc = timeOne(pl, &ms);
             if (rc) {
@@ -102,11 +105,8 @@ int autotune(Pool<T> &P, const mtgp_work_item_t *items, int nitems, void *out, v
                 break;
             }
             char line[160];
-            std::snprintf(line, sizeof line, "core=%d chunk=%lld%s grid=%s tasks=%d: %.4f ms\n",
-                          pl->core, (long long)pl->chunk,
-                          pl->overlap ? " overlap" : "",
-                          g == 0 ? "all" : g == 1 ? "7/8" : g == 2 ? "3/4" : g == 3 ? "5/8" : g == 4 ? "1/2" : "3/8",
-                          pl->ntasks, ms);
+            std::snprintf(line, sizeof line, "core=%d chunk=%lld grid=%s tasks=%d: %.4f ms\n",
+                          pl->core, (long long)pl->chunk, kGridNames[g], pl->ntasks, ms);
             rep += line;
             if (!*best || ms < best_ms) {
                 delete *best;
@@ -142,11 +142,11 @@ int autotune(Pool<T> &P, const mtgp_work_item_t *items, int nitems, void *out, v
                            : (b->split ? "k_batch32 (one word per thread, in-CTA jumps)"
                                        : "k_batch32 (one word per thread)");
         char grid[32], pre[64] = "", line[256];
-        if (b->grid > 0) std::snprintf(grid, sizeof grid, "%d CTAs", b->grid);
+        const int ctas = b->grid > 0 ? b->grid : b->auto_grid;
+        if (ctas > 0) std::snprintf(grid, sizeof grid, "%d CTAs", ctas);
         else std::snprintf(grid, sizeof grid, "all resident");
         if (b->npre)
-            std::snprintf(pre, sizeof pre, " %s k_jump_part (%d windows jumped ahead)",
-                          b->overlap ? "beside" : "after", b->npre);
+            std::snprintf(pre, sizeof pre, " after k_jump_part (%d windows jumped ahead)", b->npre);
         std::snprintf(line, sizeof line, "chosen: %s%s, chunk=%lld, grid=%s, tasks=%d: %.4f ms\n",
                       kern, pre, (long long)b->chunk, grid, b->ntasks, best_ms);
         rep += line;
