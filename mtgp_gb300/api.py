@@ -467,12 +467,11 @@ class Server:
     def replay(self, requests, arrivals):
         """Submit `requests` (a REQUEST_DTYPE array) at `arrivals` (seconds
         from now) and drain; returns the wall time in seconds.  Results of
-        requests without destination are discarded at completion.  Work queued
-        on the current stream (on the destinations) is waited for first."""
+        requests without destination are discarded at completion.  Earlier work
+        on the destinations has to be done before the call, as for submit."""
         req = np.ascontiguousarray(requests, dtype=REQUEST_DTYPE)
         arr = np.ascontiguousarray(arrivals, dtype=np.float64)
         assert len(req) == len(arr)
-        torch.cuda.current_stream().synchronize()
         wall = ctypes.c_double()
         check(lib().mtgp_server_replay(self.h, req.ctypes.data_as(ctypes.c_void_p),
                                        arr.ctypes.data_as(ctypes.c_void_p), len(arr),
