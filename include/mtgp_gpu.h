@@ -555,7 +555,8 @@ int mtgp_server_release(mtgp_server_t *s, uint64_t ticket);
 int mtgp_server_cancel(mtgp_server_t *s, uint64_t ticket);
 /* Wait until a request is done (its destination holds the result);
  * `status` receives MTGP_OK or the error it ended with (a request whose batch
- * failed may still have advanced its stream). */
+ * failed may still have advanced its stream and written part of its
+ * destination). */
 int mtgp_server_wait(mtgp_server_t *s, uint64_t ticket, double timeout_s,
                      int *status);
 /* Wait until every submitted request is done. */

@@ -131,10 +131,11 @@ inline int applyTuning(Tuning &t, const char *key, int64_t value) {
 
 // CTAs per jump, for njumps jumps made together ahead of a batched launch
 // (tuning knob jump_parts; automatic: as many as keep all the jumps' CTAs
-// resident at once, two per SM, and at most eight).  Every part makes the
-// sequence anew, so more parts than that only add work: one generator's fill
-// of 2^20 values (31 jumps) takes 36 us with 4 to 8 parts, 42 with 16; 255
-// jumps at MEXP 11213/64 take 32 us with one part, 49 with three.
+// resident at once, two per SM, and at most eight; a split fill's teams the
+// power of two below).  Every part makes the sequence anew, so more parts than
+// that only add work: one generator's fill of 2^20 values (63 jumps) takes 25
+// us with 4, 28 with one, 32 with 8; of 2^25 64-bit values (255 jumps) 118 us
+// with one, 130 with two.
 constexpr int kMaxJumpParts = 8;
 inline int jumpParts(const Tuning &t, int njumps, int sms) {
     if (t.jump_parts > 0) return (int)std::min<int64_t>(t.jump_parts, kJumpUnits);

@@ -12,9 +12,8 @@ namespace {
 // kept on the device for the chunk length; then one batched launch runs every
 // chunk from its window on the two-word core, with no jump inside it, and the
 // last chunk leaves its final window in the generator: two launches in all.
-// A 2^20-value fill takes 0.035 ms this way (0.41 ms on one CTA), 2^25 values
-// 0.09 ms.  Smaller fills,
-// and fills issued while the stream is being captured, run on one CTA.  The
+// A 2^20-value fill takes 25 us this way (247 us on one CTA), 2^25 values 77 us.
+// Smaller fills, and fills issued while the stream is being captured, run on one CTA.  The
 // first split fill of a parameter set also computes its characteristic
 // polynomial and jump tables (tens of milliseconds, and a device
 // synchronisation), and a new chunk length its chunk polynomials.
@@ -23,10 +22,10 @@ constexpr int64_t kMaxFillChunks = 4096;
 
 // Chunk length of a split fill of n values: the power of two nearest to
 // 20 sqrt(n) for MEXP 11213 (more chunks cost more jumps, longer ones a longer
-// run: 2^20 32-bit values take 34.8 us with 2^14, 36.1 with 2^15, 41.1 with
-// 2^16; 2^24 take 90.3 with 2^15, 66.0 with 2^16, 69.9 with 2^17), scaled by
+// run: 2^20 32-bit values take 28.1 us with 2^13, 24.5 with 2^14, 25.9 with
+// 2^15; 2^24 take 79.2 with 2^15, 55.5 with 2^16, 58.8 with 2^17), scaled by
 // mexp / 11213 (a jump's correlation grows with mexp^2, so the best length
-// grows with mexp: 2^25 at MEXP 23209, 249 us with 2^16, 124 with 2^18).
+// grows with mexp: 2^25 at MEXP 23209, 235 us with 2^16, 109 with 2^18).
 int64_t singleChunk(size_t n, int mexp) {
     const double t = 20.0 * (mexp / 11213.0) * std::sqrt((double)n);
     int64_t c = 1;
