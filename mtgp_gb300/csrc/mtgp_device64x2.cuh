@@ -34,7 +34,6 @@ struct Geo64x2 {
     static constexpr int BUF = K * PW;           // 64-bit words of the buffer
     static constexpr int STEP = W / K;           // plane offset advance per sub-step
     static constexpr int S = (B - N - (K - 1)) / W;  // sub-steps per segment
-    static constexpr bool kLongTail = S > 16;        // as GeoK's
     static_assert(W % (32 * K) == 0 && B % K == 0, "bad geometry");
     static_assert(S >= 2 && S * W >= N + K - 1 && S * W + N + K - 1 <= B,
                   "bad segment geometry");
@@ -205,14 +204,11 @@ struct Core64x2 {
         const int rem = (int)n;
         if (rem > 0) {
             const int subs = (rem + W - 1) / W;
-            for (int k = 0; k < subs; k++) {
+            for (int k = 0; k < subs; k++)
                 sub(buf, I, k, L, mul1, P, [&] {
-                    if (G::kLongTail && k > 0) emit<false>(P, olo, ohi, o + (k - 1) * W, K);
+                    if (k > 0) emit<false>(P, olo, ohi, o + (k - 1) * W, K);
                 });
-                if (!G::kLongTail) emit<true>(P, olo, ohi, o + k * W, rem - k * W - K * t);
-            }
-            if (G::kLongTail)
-                emit<true>(P, olo, ohi, o + (subs - 1) * W, rem - (subs - 1) * W - K * t);
+            emit<true>(P, olo, ohi, o + (subs - 1) * W, rem - (subs - 1) * W - K * t);
         }
         if (phase + rem != 0) move(buf, phase + rem, 0);
     }
